@@ -13,13 +13,13 @@ from .config import ModelConfig
 
 # CUDA translation units of a family, for callers that build no more than they run (None: the whole library)
 KERNEL_UNITS = {
-    "zokuvik": ("elementwise", "gemm_tcgen05", "gemm_simt", "group_norm", "latent_attention", "latent_decode", "latent_prefill",
+    "zokuvik": ("elementwise", "gemm_tcgen05", "gemm_prompt", "gemm_simt", "group_norm", "latent_attention", "latent_decode", "latent_prefill",
                 "delta_rule", "state_scan"),
-    "sepedra": ("elementwise", "gemm_tcgen05", "gemm_simt", "group_norm", "attention", "kv_attention", "short_conv", "latent_prefill", "rglru", "moe",
+    "sepedra": ("elementwise", "gemm_tcgen05", "gemm_prompt", "gemm_simt", "group_norm", "attention", "kv_attention", "short_conv", "latent_prefill", "rglru", "moe",
                 "moe_dense"),
-    "kegorax": ("elementwise", "gemm_tcgen05", "gemm_simt", "group_norm", "attention", "kv_attention", "short_conv", "latent_prefill",
+    "kegorax": ("elementwise", "gemm_tcgen05", "gemm_prompt", "gemm_simt", "group_norm", "attention", "kv_attention", "short_conv", "latent_prefill",
                 "linear_state", "state_scan", "moe", "moe_dense"),
-    "fekolorn": ("elementwise", "gemm_tcgen05", "gemm_simt", "hyper_streams", "poly_norm", "attention", "kv_attention", "short_conv",
+    "fekolorn": ("elementwise", "gemm_tcgen05", "gemm_prompt", "gemm_simt", "hyper_streams", "poly_norm", "attention", "kv_attention", "short_conv",
                  "latent_prefill", "linear_state", "state_scan"),
 }
 

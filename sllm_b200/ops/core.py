@@ -139,6 +139,37 @@ def _gemm_plan(m: int, n: int, k_blocks: int):
     return False, 128, 1, 5
 
 
+# Cycles of one 128-byte K block of a pair's tile by its columns (csrc/gemm_prompt.cu), measured with the machine full: bf16 is held
+# by L2 below 256 columns, E4M3 by the promotion of every block's sums
+_PROMPT_BLOCK = {False: {64: 520, 128: 540, 256: 700}, True: {64: 830, 128: 1060, 256: 2050}}
+
+
+def _prompt_tile(m: int, n: int, scaled: bool) -> int:
+    """Columns of a tile of the prompt product: the fewest cycles over the waves of 74 CTA pairs, 256 rows a pair.  Narrow tiles
+    spread few rows over more pairs (130 x 4096 x 4096: 25 us with 64 columns, 31 with 256), wide ones reuse their operands
+    (8192 x 28672 x 4096: 2310 us with 64, 1190 with 256)."""
+    cost = _PROMPT_BLOCK[scaled]
+    return min((256, 128, 64), key=lambda bn: (((m + 255) // 256 * ((n + bn - 1) // bn) + 73) // 74) * cost[bn])
+
+
+def _linear_prompt(x: torch.Tensor, w: LinearWeight, y: torch.Tensor, scale_x: Optional[torch.Tensor], residual: Optional[torch.Tensor],
+                   act: Optional[str], act_arg: float) -> None:
+    from ..core.types import reject_aliasing
+    m, n, k = x.shape[0], w.out_features, w.in_features
+    reject_aliasing(y, {"x": x, "w": w.w, "scale_x": scale_x, "scale_w": w.scale_t, "residual": residual}, may_equal=("residual",))
+    scaled = scale_x is not None
+    epilogue = 1 if residual is not None else {None: 0, "relu_sq": 2, "softcap": 3}[act]
+    bn = _prompt_tile(m, n, scaled)
+    if _lib.audit_enabled():
+        _lib.record_dispatch("linear", "gemm_prompt_kernel", m=m, n=n, k=k, kind=w.kind, bn=bn,
+                             grid=[min(148, 2 * ((m + 255) // 256) * ((n + bn - 1) // bn))])
+    rc = _lib.kernels().sllm_gemm_prompt(_p(x), _p(w.w), _p(y), _p(scale_x), _p(w.scale_t) if scaled else None, _p(residual), m, n, k,
+                                         x.stride(0), y.stride(0), scale_x.stride(0) if scaled else 0,
+                                         w.scale_t.stride(0) if scaled else 0, epilogue, act_arg, bn, _p(workspace(x.device).status),
+                                         _stream())
+    _lib.check(rc, "gemm_prompt")
+
+
 def gemm_raw(a: torch.Tensor, b: torch.Tensor, y: torch.Tensor, *, scale_a=None, scale_b=None, residual=None,
              transpose_out: bool, bn: int, splits: int, stages: int) -> None:
     """Direct access to the tcgen05 kernel: D[a_row, b_row] = sum_k A[a_row, k] B[b_row, k]."""
@@ -213,6 +244,12 @@ def linear(x, w: LinearWeight, residual: Optional[torch.Tensor] = None, act: Opt
     else:
         k_blocks = (w.in_features + 63) // 64
     y = torch.empty((m, n), dtype=torch.float32 if out_fp32 else torch.bfloat16, device=xd.device)
+    if w.kind != "fp8" and m > 1 and x.stride(0) != x.shape[1] and residual is not None:
+        raise ValueError("a product with a residual takes contiguous rows")
+    # prompts: pairs of CTAs; it stores whole 16-byte units of bf16 rows, other widths and fp32 sums stay with the general kernel
+    if m > 128 and n % 8 == 0 and not out_fp32 and (residual is None or (residual.is_contiguous() and residual.dtype == torch.bfloat16)):
+        _linear_prompt(x.data if w.kind == "fp8" else x, w, y, x.scale if w.kind == "fp8" else None, residual, act, act_arg)
+        return y
     swap, bn, splits, stages = _gemm_plan(m, n, k_blocks)
     if _lib.audit_enabled():
         _lib.record_dispatch("linear", "gemm_tcgen05_kernel", m=m, n=n, k=w.in_features, kind=w.kind, swap_ab=swap, bn=bn,
@@ -227,8 +264,6 @@ def linear(x, w: LinearWeight, residual: Optional[torch.Tensor] = None, act: Opt
                      bn=bn, splits=splits, stages=stages)
     else:
         strided = m > 1 and x.stride(0) != x.shape[1]
-        if strided and residual is not None:
-            raise ValueError("a product with a residual takes contiguous rows")
         if act or out_fp32 or strided:
             a, b = (w.w, x) if swap else (x, w.w)
             wsp = workspace(xd.device)

@@ -1,0 +1,59 @@
+"""The product of many rows (csrc/gemm_prompt.cu) at the edges of its tiles, against fp64."""
+import pytest
+import torch
+
+from sllm_b200 import ops
+from sllm_b200.ops import core
+from sllm_b200.ops.core import LinearWeight
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _operands(m, n, k, scaled, seed):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    x = torch.randn(m, k, generator=g, device=DEV).bfloat16()
+    w = (torch.randn(n, k, generator=g, device=DEV) * 0.05).bfloat16()
+    r = torch.randn(m, n, generator=g, device=DEV).bfloat16()
+    if not scaled:
+        return x, LinearWeight("dense", w), x.double(), w.double(), r
+    xq, wq = ops.quant_fp8(x), ops.quant_fp8(w)
+    real = lambda q: q.data.view(torch.float8_e4m3fn).double() * q.scale.t().double().repeat_interleave(128, 1)[:, :k]
+    return xq, LinearWeight("fp8", wq.data, wq.scale), real(xq), real(wq), r
+
+
+def _close(got, want, xf, wf):
+    # fp32 sums in any order (k 2^-23 of the sum of magnitudes) and one rounding to bf16
+    bound = want.abs() * 2.0 ** -8 + (xf.abs() @ wf.abs().t()) * (xf.shape[1] * 2.0 ** -23) + 1e-30
+    assert ((got.double() - want).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("scaled", [False, True])
+@pytest.mark.parametrize("m,n,k", [(129, 8, 64), (255, 264, 128), (257, 72, 208), (385, 520, 1040), (512, 256, 4096), (1030, 136, 640)])
+@pytest.mark.parametrize("bn", [64, 128, 256])
+def test_tiles(monkeypatch, scaled, m, n, k, bn):
+    monkeypatch.setattr(core, "_prompt_tile", lambda *a: bn)
+    x, w, xf, wf, r = _operands(m, n, k, scaled, m + n + k)
+    want = xf @ wf.t()
+    _close(ops.linear(x, w), want, xf, wf)
+    _close(ops.linear(x, w, r), want + r.double(), xf, wf)
+    assert ops.device_status(torch.device(DEV, 0)) == 0
+
+
+def test_many_tiles_per_pair():
+    """More tiles than pairs: accumulators, stages and scale chunks wrap around across tiles."""
+    for scaled in (False, True):
+        x, w, xf, wf, r = _operands(2600, 8200, 320, scaled, 5)
+        _close(ops.linear(x, w, r), xf @ wf.t() + r.double(), xf, wf)
+
+
+def test_activations_and_strided_rows():
+    x, w, xf, wf, _ = _operands(300, 200, 256, False, 9)
+    want = xf @ wf.t()
+    relu = ops.linear(x, w, act="relu_sq").double()
+    assert ((relu - want.clamp(min=0) ** 2).abs() <= (want.clamp(min=0) ** 2) * 2.0 ** -7 + 1e-3).all()
+    cap = ops.linear(x, w, act="softcap", act_arg=2.0).double()
+    assert ((cap - 2.0 * torch.tanh(want / 2.0)).abs() <= 2.0 ** -7).all()
+    wide = torch.zeros(300, 512, device=DEV, dtype=torch.bfloat16)
+    wide[:, 8:264] = x
+    _close(ops.linear(wide[:, 8:264], w), want, xf, wf)
