@@ -16,6 +16,7 @@ from . import _lib
 P, I, F = C.c_void_p, C.c_int, C.c_float
 _SIGS = {
     "sllm_gdn_conv_silu": (I, [P, P, P, P, P, P, I, I, I, I, P]),
+    "sllm_gdn_conv_silu_prompt": (I, [P, P, P, P, P, P, I, I, I, I, I, P]),
     "sllm_gdn_recurrent": (I, [P, P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, P]),
     "sllm_gdn_recurrent_prompt": (I, [P] * 11 + [I] * 7 + [P, C.c_longlong, P]),
     "sllm_qk_headnorm": (I, [P, I, I, I, I, I, P, P, F, I, P]),
@@ -55,6 +56,13 @@ def conv_silu(x: torch.Tensor, w: torch.Tensor, state: torch.Tensor, row_off: to
     if x.stride(1) != 1:
         x = x.contiguous()
     y = torch.empty((t, width), dtype=x.dtype, device=x.device)       # x may be a column slice of a wider matrix
+    if (t >= PROMPT_FORM_MIN_ROWS_PER_SEQUENCE * slots.numel() and prompt_form_enabled() and width % 2 == 0 and x.stride(0) % 2 == 0
+            and (x.data_ptr() | state.data_ptr()) % 4 == 0 and t <= 65535 * 32):
+        # many rows per sequence: rows in parallel, channels in pairs
+        rc = _k().sllm_gdn_conv_silu_prompt(_p(x), _p(w), _p(state), _p(y), _p(row_off), _p(slots), slots.numel(), t, width, taps,
+                                            x.stride(0), _stream())
+        _lib.check(rc, "gdn_conv_silu_prompt")
+        return y
     rc = _k().sllm_gdn_conv_silu(_p(x), _p(w), _p(state), _p(y), _p(row_off), _p(slots), slots.numel(), width, taps,
                                  x.stride(0), _stream())
     _lib.check(rc, "gdn_conv_silu")
