@@ -69,6 +69,7 @@ struct GpParams {
   int ldy, ld_sx, ld_sw;
   int epilogue;                             // 0 store, 1 add residual, 2 square of relu, 3 soft cap
   float act_arg;
+  const float* alpha;                       // optional factor of the sums (bf16 operands)
   const float *scale_x, *scale_w;           // [num_kb, ld]
   const __nv_bfloat16* residual;            // [m, ldy]
   int* status;
@@ -338,6 +339,7 @@ gemm_prompt_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
         }
       }
     } else {
+      const float alpha = p.alpha ? *p.alpha : 1.f;
       for (int t = pair; ok && t < tiles; t += pairs, ++acc) {
         int tm, tn;
         gp_tile(p, t, tm, tn);
@@ -354,7 +356,7 @@ gemm_prompt_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
             tmem_ld16(lane_addr + (acc % S::kAcc) * BN + c * 64 + i * 16, r);
             tmem_wait_regs(r);
 #pragma unroll
-            for (int j = 0; j < 16; ++j) v[i * 16 + j] = __uint_as_float(r[j]);
+            for (int j = 0; j < 16; ++j) v[i * 16 + j] = __uint_as_float(r[j]) * alpha;
           }
           if (c == S::kCols / 64 - 1) {                    // all of it is in registers
             tc_fence_before();
@@ -410,18 +412,19 @@ using namespace sllm;
 
 // x [m, k] (row stride ldx elements), w [n, k] contiguous, y [m, n] bf16 (row stride ldy): bf16 operands, or with scale_x / scale_w
 // E4M3 and scales [ceil(k / 128), ld].  epilogue: 0 store, 1 add residual [m, ldy], 2 square of relu, 3 act_arg tanh(. / act_arg).
-// bn: columns of a pair's tile, 64, 128 or 256.  n and ldy are multiples of 8, rows of x and w of 16 bytes.
+// alpha: optional device scalar that multiplies the sums of bf16 operands.  bn: columns of a pair's tile, 64, 128 or 256.  n and ldy are multiples of 8, rows of x and w of 16 bytes.
 SLLM_EXPORT int sllm_gemm_prompt(const void* x, const void* w, void* y, const float* scale_x, const float* scale_w, const void* residual,
-                                 int m, int n, int k, long long ldx, int ldy, int ld_sx, int ld_sw, int epilogue, float act_arg, int bn,
-                                 int* status, void* stream) {
+                                 int m, int n, int k, long long ldx, int ldy, int ld_sx, int ld_sw, int epilogue, float act_arg,
+                                 const float* alpha, int bn, int* status, void* stream) {
   if (!x || !w || !y || m <= 0 || n <= 0 || k <= 0 || ldx < k || ldy < n || epilogue < 0 || epilogue > 3 || (epilogue == 1) != (residual != nullptr))
     return SLLM_ERR_INVALID_ARGUMENT;
+  if (alpha && scale_x) return SLLM_ERR_UNSUPPORTED_SHAPE;
   if (!scale_x != !scale_w || (scale_x && (ld_sx < m || ld_sw < n))) return SLLM_ERR_INVALID_ARGUMENT;
   if ((n & 7) || (ldy & 7) || (reinterpret_cast<uintptr_t>(residual) & 15)) return SLLM_ERR_ALIGNMENT;
   const bool scaled = scale_x != nullptr;
   GpParams p = {};
   p.m = m; p.n = n; p.num_kb = scaled ? (k + 127) / 128 : (k + 63) / 64;
-  p.ldy = ldy; p.ld_sx = ld_sx; p.ld_sw = ld_sw; p.epilogue = epilogue; p.act_arg = act_arg;
+  p.ldy = ldy; p.ld_sx = ld_sx; p.ld_sw = ld_sw; p.epilogue = epilogue; p.act_arg = act_arg; p.alpha = alpha;
   p.scale_x = scale_x; p.scale_w = scale_w; p.residual = static_cast<const __nv_bfloat16*>(residual); p.status = status;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   switch (bn) {

@@ -60,6 +60,7 @@ struct W4Params {
   int n_valid;         // output features per group
   int k_chunks;        // K_pad / 128
   int groups;
+  int tok_tiles;       // token tiles of the largest possible group
   int scale_bytes;     // per row per chunk: 4 (MXFP4) or 8 (NVFP4)
   int stages;
   int splits;
@@ -148,13 +149,43 @@ gemm_w4_kernel(const __grid_constant__ CUtensorMap tm_x, const W4Params p) {
   constexpr uint32_t kTmemCols = kW4Issuers * BN < 32 ? 32 : kW4Issuers * BN;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int row_tile = blockIdx.x, g = blockIdx.y;
-  if (p.tok_off) pdl_wait();      // the group offsets come from the routing kernels just before this one
-  const int tt = blockIdx.z / p.splits, split = blockIdx.z % p.splits;
+  const int row_tile = blockIdx.x, split = blockIdx.z;
+  int g = 0, tt = blockIdx.y;
+  if (p.tok_off && p.tok_tiles == 1) {               // one tile holds any group: a decode step
+    pdl_wait();
+    g = blockIdx.y;
+    tt = 0;
+  } else if (p.tok_off) {
+    // Token tile blockIdx.y of those that the groups really have, counted over the groups in order (every warp counts for itself).
+    // A tile for every group and every token it could hold had been 363 000 CTAs for 2000 tokens of 128 experts x 45 row tiles,
+    // 98 % of them empty; the products of two such layers took 14.7 ms, now 4.7.
+    pdl_wait();                   // the group offsets come from the routing kernels just before this one
+    int before = 0;
+    bool found = false;
+    for (int base = 0; base < p.groups && !found; base += 32) {
+      const int e = base + lane;
+      const int n = e < p.groups ? (p.tok_off[e + 1] - p.tok_off[e] + BN - 1) / BN : 0;
+      int sum = n;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, sum, o);
+        if (lane >= o) sum += v;
+      }
+      const unsigned hit = __ballot_sync(0xffffffffu, static_cast<int>(blockIdx.y) < before + sum);
+      if (hit) {
+        const int l = __ffs(hit) - 1;
+        g = base + l;
+        tt = blockIdx.y - before - __shfl_sync(0xffffffffu, sum - n, l);
+        found = true;
+      }
+      before += __shfl_sync(0xffffffffu, sum, 31);
+    }
+    if (!found) return;           // uniform: the grid has room for every way to divide the tokens
+  }
   const int t_begin = (p.tok_off ? p.tok_off[g] : 0) + tt * BN;
   const int t_end_g = p.tok_off ? p.tok_off[g + 1] : p.total_tokens;
   const int count = min(BN, t_end_g - t_begin);
-  if (count <= 0) return;                                   // uniform: an expert without tokens reads nothing
+  if (count <= 0) return;
   const int per = (p.k_chunks + p.splits - 1) / p.splits;
   const int c0 = split * per;
   const int nk = max(0, min(per, p.k_chunks - c0));
@@ -390,7 +421,7 @@ gemm_w4_kernel(const __grid_constant__ CUtensorMap tm_x, const W4Params p) {
     if (p.splits > 1) {
       __threadfence();
       asm volatile("bar.sync 1, 128;" ::: "memory");
-      const int tile_id = (g * gridDim.x + row_tile) * (gridDim.z / p.splits) + tt;
+      const int tile_id = (g * gridDim.x + row_tile) * p.tok_tiles + tt;
       if (threadIdx.x == 64) {
         const int prev = atomicAdd(&p.counters[tile_id], 1);
         bars->is_last = (prev == p.splits - 1);
@@ -416,6 +447,36 @@ gemm_w4_kernel(const __grid_constant__ CUtensorMap tm_x, const W4Params p) {
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, kTmemCols);
+  }
+}
+
+// Rows [row0, row0 + rows) of a dense weight as bf16 [rows, k]: codes times block scales, exact (at most five significant bits); the
+// tensor scale stays with the product.  Prompts multiply the expanded matrix on CTA pairs (gemm_prompt.cu): the conversion above is
+// repeated by every token tile.  The 16 matrices of four layers (d 4096, ffn 14336) on 1076 rows: 5627 us there, 1673 + 399 for the
+// expansion here.
+// grid (K chunks, row tiles), 256 threads: a thread takes eight codes of one word, 16 lanes a row's 256 bytes.
+template <int kFmt>
+__global__ void __launch_bounds__(256)
+w4_expand_kernel(const uint8_t* __restrict__ tiles, __nv_bfloat16* __restrict__ out, int row0, int rows, int k, int k_chunks) {
+  pdl_wait();
+  pdl_trigger();
+  constexpr int kScaleBytes = kFmt == 0 ? 4 : 8;
+  const uint8_t* t = tiles + (static_cast<size_t>(row0 / kW4Rows + blockIdx.y) * k_chunks + blockIdx.x) * (kW4PackedBytes + kW4Rows * kScaleBytes);
+  uint32_t words[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) words[j] = reinterpret_cast<const uint32_t*>(t)[threadIdx.x + 256 * j];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const int i = threadIdx.x + 256 * j, r = i >> 4, c = i & 15, row = blockIdx.y * kW4Rows + r, col = blockIdx.x * kW4Chunk + c * 8;
+    const uint32_t f = block_factor<kFmt>(t[kW4PackedBytes + r * kScaleBytes + c / (kFmt == 0 ? 4 : 2)]);
+    uint4 o;
+    uint32_t* x = reinterpret_cast<uint32_t*>(&o);
+#pragma unroll
+    for (int pr = 0; pr < 4; ++pr) {
+      const uint32_t y = words[j] >> (4 * pr);
+      x[pr] = bf16x2_mul(bf16x2_mul(((y & 0x00070007u) << 6) | ((y & 0x00080008u) << 12), f), 0x47804780u);   // times 2^16
+    }
+    if (row < rows && col < k) *reinterpret_cast<uint4*>(out + static_cast<size_t>(row) * k + col) = o;
   }
 }
 
@@ -477,6 +538,10 @@ static int gemm_w4_impl(const void* wtiles, const float* tensor_scale, const voi
   const int row_tiles = n_rows / kW4Rows;
   const int tok_tiles = (max_group_tokens + bn - 1) / bn;
   if (static_cast<long long>(tok_tiles) * splits > 65535 || groups > 65535) return SLLM_ERR_UNSUPPORTED_SHAPE;
+  // grouped: at most a partly filled tile per group on top of the tokens' full ones
+  long long tiles = static_cast<long long>(tok_tiles) * groups;
+  if (tok_off && tiles > total_tokens / bn + groups) tiles = total_tokens / bn + groups;
+  if (tiles > 65535) return SLLM_ERR_UNSUPPORTED_SHAPE;
   if (splits > 1) {
     if (!ws || !counters) return SLLM_ERR_INVALID_ARGUMENT;
     if (ws_floats < static_cast<long long>(splits) * total_tokens * n_valid ||
@@ -494,7 +559,8 @@ static int gemm_w4_impl(const void* wtiles, const float* tensor_scale, const voi
   p.tok_scale = tok_scale; p.residual = static_cast<const __nv_bfloat16*>(residual);
   p.y = static_cast<__nv_bfloat16*>(y); p.ws = ws; p.counters = counters; p.status = status;
   p.row_ptr = row_ptr;
-  dim3 grid(row_tiles, groups, tok_tiles * splits);
+  p.tok_tiles = tok_tiles;
+  dim3 grid(row_tiles, static_cast<unsigned>(tiles), splits);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
 #define SLLM_W4_CASE(BNV)                                                                      \
   case BNV:                                                                                    \
@@ -531,4 +597,17 @@ SLLM_EXPORT int sllm_gemm_w4_scatter(const void* wtiles, const float* tensor_sca
   return gemm_w4_impl(wtiles, tensor_scale, x, nullptr, nullptr, tok_off, tok_scale, fmt, groups, n_rows, n_valid, k_pad, k,
                       ldx, total_tokens, max_group_tokens, n_valid, bn, splits, stages, ws, ws_floats, counters, n_counters,
                       status, stream, row_ptr);
+}
+
+// out [rows, k] bf16 from rows row0 .. row0 + rows - 1 of a dense tiled weight; row0 a multiple of 128, k of 8.
+SLLM_EXPORT int sllm_w4_expand(const void* wtiles, void* out, int fmt, int n_rows, int k_pad, int row0, int rows, int k, void* stream) {
+  if (!wtiles || !out || (fmt != 0 && fmt != 1) || n_rows <= 0 || (n_rows % kW4Rows) || k_pad <= 0 || (k_pad % kW4Chunk) || k <= 0 ||
+      k > k_pad || row0 < 0 || (row0 % kW4Rows) || rows <= 0 || row0 + rows > n_rows || rows > 65535 * kW4Rows)
+    return SLLM_ERR_INVALID_ARGUMENT;
+  if ((k & 7) || (reinterpret_cast<uintptr_t>(out) & 15) || (reinterpret_cast<uintptr_t>(wtiles) & 3)) return SLLM_ERR_ALIGNMENT;
+  return launch_kernel(fmt == 0 ? w4_expand_kernel<0> : w4_expand_kernel<1>, dim3(k_pad / kW4Chunk, (rows + kW4Rows - 1) / kW4Rows),
+                       dim3(256), 0, static_cast<cudaStream_t>(stream), 1u, static_cast<const uint8_t*>(wtiles),
+                       static_cast<__nv_bfloat16*>(out), row0, rows, k, k_pad / kW4Chunk) == cudaSuccess
+             ? SLLM_OK
+             : SLLM_ERR_CUDA;
 }

@@ -242,6 +242,38 @@ def _bn_for(tokens: int) -> int:
     return 16 if tokens <= 16 else 32 if tokens <= 32 else 64 if tokens <= 64 else 128
 
 
+EXPAND_ELEMENTS = 1 << 27      # of an expanded weight at a time (256 MB)
+
+
+def _expandable(x, w: W4Weight, residual, tok_off, tok_scale, row_ptr) -> bool:
+    """Whether a product expands its weight to bf16 first: dense, more rows than the decode kernels' tiles hold, whole 16-byte units."""
+    return (x.shape[0] > 128 and w.groups == 1 and tok_off is None and tok_scale is None and row_ptr is None and x.dtype == torch.bfloat16
+            and w.k % 8 == 0 and w.n % 8 == 0 and x.stride(1) == 1 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0
+            and (residual is None or (residual.is_contiguous() and residual.dtype == torch.bfloat16 and residual.data_ptr() % 16 == 0)))
+
+
+def _linear_expanded(x: torch.Tensor, w: W4Weight, residual: Optional[torch.Tensor]) -> torch.Tensor:
+    """Rows of the weight are expanded to bf16 (exact) and multiplied on CTA pairs, EXPAND_ELEMENTS of them at a time."""
+    from .core import _p, _prompt_tile, _stream, workspace
+    t, k = x.shape
+    y = torch.empty((t, w.n), dtype=torch.bfloat16, device=x.device)
+    step = max(256, EXPAND_ELEMENTS // k // 256 * 256)
+    dense = torch.empty((min(step, w.n), k), dtype=torch.bfloat16, device=x.device)
+    lib, status = _lib.kernels(), _p(workspace(x.device).status)
+    for r0 in range(0, w.n, step):
+        rows = min(step, w.n - r0)
+        rc = lib.sllm_w4_expand(_p(w.tiles), _p(dense), 0 if w.fmt == "mxfp4" else 1, w.n_rows, w.k_pad, r0, rows, k, _stream())
+        _lib.check(rc, "w4_expand")
+        bn = _prompt_tile(t, rows, False)
+        if _lib.audit_enabled():
+            _lib.record_dispatch("linear_w4", "gemm_prompt_kernel", fmt=w.fmt, tokens=t, n=rows, k=k, groups=1, grouped=False, bn=bn)
+        res = None if residual is None else residual[:, r0:]
+        rc = lib.sllm_gemm_prompt(_p(x), _p(dense), _p(y[:, r0:]), None, None, _p(res), t, rows, k, x.stride(0), w.n, 0, 0,
+                                  0 if residual is None else 1, 0.0, _p(w.tensor_scale), bn, status, _stream())
+        _lib.check(rc, "gemm_prompt")
+    return y
+
+
 def linear_w4(x: torch.Tensor, w: W4Weight, residual: Optional[torch.Tensor] = None, tok_off: Optional[torch.Tensor] = None,
               tok_scale: Optional[torch.Tensor] = None, max_group_tokens: Optional[int] = None, splits: int = 0,
               row_ptr: Optional[torch.Tensor] = None) -> Optional[torch.Tensor]:
@@ -280,10 +312,14 @@ def linear_w4(x: torch.Tensor, w: W4Weight, residual: Optional[torch.Tensor] = N
                                                                P, L, P, I, P, P]))
     if w.groups > 1 and tok_off is None:
         raise ValueError("grouped weights need token offsets")
+    if splits <= 0 and _expandable(x, w, residual, tok_off, tok_scale, row_ptr):
+        return _linear_expanded(x, w, residual)
     x = x.contiguous() if x.stride(1) != 1 or x.stride(0) % 8 else x
     y = torch.empty((t, w.n), dtype=torch.bfloat16, device=x.device)
     mgt = max_group_tokens or t
-    bn = _bn_for(mgt if tok_off is None else min(mgt, 32))
+    # grouped: a tile that holds the mean of the groups with a quarter to spare, so that few groups convert their weights twice
+    # (62 rows for each of 128 experts, two layers: 13.1 ms in tiles of 16, 10.1 of 32, 8.2 of 64, 7.85 of 128)
+    bn = _bn_for(mgt if tok_off is None else min(mgt, 5 * t // (4 * w.groups)))
     k_chunks = w.k_pad // 128
     if splits <= 0:
         ctas = (w.n_rows // 128) * (w.groups if tok_off is None else max(1, min(w.groups, t))) * ((min(mgt, t) + bn - 1) // bn)

@@ -1,0 +1,49 @@
+"""4-bit weights with many rows: expanded dense matrices and the token tiles of routed experts."""
+import numpy as np
+import pytest
+import torch
+
+from sllm_b200 import ops
+from sllm_b200.ops import w4
+from sllm_b200.ops.w4 import W4Weight, linear_w4
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+@pytest.mark.parametrize("fmt", ["mxfp4", "nvfp4"])
+@pytest.mark.parametrize("t,n,k", [(129, 136, 200), (260, 640, 384), (300, 1032, 128)])
+def test_expanded_products(monkeypatch, fmt, t, n, k):
+    g = torch.Generator(device=DEV).manual_seed(t)
+    weight = W4Weight.quantize_device(fmt, torch.randn(n, k, generator=g, device=DEV) * 0.05)
+    real = weight.dequantized(0).double().to(DEV)
+    x = torch.randn(t, k, generator=g, device=DEV).bfloat16()
+    r = torch.randn(t, n, generator=g, device=DEV).bfloat16()
+    for elements in (w4.EXPAND_ELEMENTS, 256 * k):                 # at once, and in pieces of 256 rows
+        monkeypatch.setattr(w4, "EXPAND_ELEMENTS", elements)
+        for res in (None, r):
+            want = x.double() @ real.t() + (0 if res is None else res.double())
+            bound = want.abs() * 2.0 ** -8 + (x.double().abs() @ real.abs().t()) * (k * 2.0 ** -23)
+            assert ((linear_w4(x, weight, residual=res).double() - want).abs() <= bound).all()
+    assert ops.device_status(torch.device(DEV, 0)) == 0
+
+
+@pytest.mark.parametrize("counts", [[0, 0, 300], [17, 0, 64, 65, 1, 128, 0, 129], [3] * 70, [0] * 40 + [200, 5]])
+def test_token_tiles_of_experts(counts):
+    g = torch.Generator(device=DEV).manual_seed(len(counts))
+    e, t, n, k = len(counts), sum(counts), 136, 256
+    weight = W4Weight.quantize_device("mxfp4", torch.randn(e, n, k, generator=g, device=DEV) * 0.05)
+    off = torch.tensor([0] + list(np.cumsum(counts)), dtype=torch.int32, device=DEV)
+    x = torch.randn(t, k, generator=g, device=DEV).bfloat16()
+    scale = torch.rand(t, generator=g, device=DEV)
+    want, size = torch.zeros(t, n, dtype=torch.double, device=DEV), torch.zeros(t, n, dtype=torch.double, device=DEV)
+    for i in range(e):
+        a, b = int(off[i]), int(off[i + 1])
+        if b > a:
+            real = weight.dequantized(i).double().to(DEV)
+            want[a:b] = x[a:b].double() @ real.t() * scale[a:b, None].double()
+            size[a:b] = x[a:b].double().abs() @ real.abs().t() * scale[a:b, None].double()
+    for splits in (0, 1, 2):
+        got = linear_w4(x, weight, tok_off=off, tok_scale=scale, max_group_tokens=t, splits=splits).double()
+        assert ((got - want).abs() <= want.abs() * 2.0 ** -8 + size * (k * 2.0 ** -23)).all()
+    assert ops.device_status(torch.device(DEV, 0)) == 0
