@@ -85,9 +85,10 @@ int sllm_decode_attention_tc(const void* q, int q_ld, const void* k_pages, const
                              void* stream);
 
 /* prefill_attention.cu */
+int sllm_prefill_tile_rows(int hq, int hkv, int hd);
 int sllm_prefill_attention(const void* qkv, int total_tokens, int qkv_ld, const int* tiles, int num_tiles, int hq,
-                           int hkv, int hd, float sm_scale, void* out_bf16, void* out_fp8, float* out_scale,
-                           int ld_scale, int* status, void* stream);
+                           int hkv, int hd, int window, float sm_scale, const float* sinks, void* out_bf16,
+                           void* out_fp8, float* out_scale, int ld_scale, int* status, void* stream);
 
 /* comm.cu */
 int sllm_symm_alloc(long long bytes, void** dev_ptr, unsigned char* handle64);

@@ -235,7 +235,8 @@ class Qwen35Model:
                 qkv = G.qk_headnorm(qkv, self.hq, self.hkv, hd, lw.q_norm, lw.k_norm, cfg.rms_eps, True)
                 q = ops.rope_kv_append(qkv, b.positions, b.seq_index, b.block_table, kv, self.hq, self.hkv, hd, cfg.rope_theta,
                                        cfg.rotary_dim)
-                a = ops.paged_attention(q, kv, b.block_table, b.seq_index, b.kv_lens, self.hq, self.hkv, hd, max_kv=b.max_kv)
+                # prompts on the tensor cores; an FP8 output projection quantises the rows, which keep the order of sums they had
+                a = ops.attention(q, kv, b, self.hq, self.hkv, hd, qkv=qkv if lw.o.kind != "fp8" else None)
                 if lw.gate is not None:
                     a = ops.elementwise("sigmoid_mul", a.contiguous(), ops.linear(x, lw.gate))
                 h = self.tp.row_linear(a, lw.o, h)

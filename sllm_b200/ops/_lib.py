@@ -187,7 +187,8 @@ _KERNEL_SIGNATURES = {
     "sllm_gemm_set_cluster_split": (None, [I]),
     "sllm_decode_attention_tc": (I, [P, I, P, P, P, P, F, F, P, I, P, P, I, I, I, I, I, I, F, P, P, P, I, P, I, P, L,
                                       P, I, P, P]),
-    "sllm_prefill_attention": (I, [P, I, I, P, I, I, I, I, F, P, P, P, I, P, P]),
+    "sllm_prefill_tile_rows": (I, [I, I, I]),
+    "sllm_prefill_attention": (I, [P, I, I, P, I, I, I, I, I, F, P, P, P, P, I, P, P]),
     "sllm_paged_attention_workspace_floats": (L, [I, I, I, I, I]),
     "sllm_paged_attention": (I, [P, I, P, P, P, P, F, F, P, I, P, P, I, I, I, I, I, I, F, I, P, P, P, I, P, I, P, L,
                                   P, I, P, L, I, I, I, P, P, I, I, P]),

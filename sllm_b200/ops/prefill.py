@@ -1,54 +1,97 @@
-"""Tensor-core prefill attention front end (kernel in csrc/prefill_attention.cu).
+"""Tensor-core prompt attention front end (kernel in csrc/prefill_attention.cu).
 
-Used for fresh prompts (every sequence starts at position 0 and its tokens are contiguous rows of the
-packed qkv activation) with head_dim 128 and no sliding window; other cases read the paged cache.
+Sequences that start at position 0 and whose tokens are contiguous rows of the packed qkv activation, heads of 64, 128 or 256
+channels, with or without a sliding window and sinks.  In a batch that also decodes, or continues prompts, the rows of the other
+sequences read the paged cache.
 """
 from __future__ import annotations
 
 import math
+from typing import Optional
 
 import torch
 
 from . import _lib
-from .core import QTensor, _alloc_q, _p, _stream, workspace
+from .core import QTensor, _alloc_q, _p, _stream, paged_attention, workspace
 
 MIN_TOKENS = 128
 TILE = 128
 
 
-def usable(q, batch, hd, window, sinks, qkv) -> bool:
-    if not q.is_cuda or qkv is None or batch.cu_seqlens is None or sinks is not None or window:
-        return False
-    if hd != 128 or batch.max_seqlen < MIN_TOKENS or batch.cu_seqlens_host is None:
-        return False
-    return hasattr(_lib.kernels(), "sllm_prefill_attention")
+def _heads_fit(q, hd, qkv) -> bool:
+    return (q.is_cuda and qkv is not None and qkv.dtype == torch.bfloat16 and hd in (64, 128, 256) and not _lib.fake_active()
+            and qkv.stride(1) == 1 and qkv.stride(0) == qkv.shape[1])
 
 
-def build_tiles(cu_seqlens: list, device) -> torch.Tensor:
+def usable(q, batch, hd, window, sinks, qkv, quant_out: bool = False) -> bool:
+    """Whether all rows of the batch take the kernel.  Results that are quantised to E4M3 are kept as they have been, since a last
+    bit's difference moves them by a sixteenth: with a window or sinks they come from the pages."""
+    if quant_out and (window or sinks is not None):
+        return False
+    return _heads_fit(q, hd, qkv) and batch.cu_seqlens_host is not None and batch.max_seqlen >= MIN_TOKENS
+
+
+def fresh_part(q, batch, hd, qkv) -> Optional[tuple]:
+    """(sequences that take the kernel, [lo, hi) runs of the other rows) of a batch that mixes prompts with running requests, or
+    None where no prompt of MIN_TOKENS starts in it."""
+    if not _heads_fit(q, hd, qkv) or batch.row_off_host is None or batch.starts_host is None or batch.row_off_host[-1] != q.shape[0]:
+        return None
+    if "fresh" not in batch.plans:
+        off, fresh, rest = batch.row_off_host, [], []
+        for i, start in enumerate(batch.starts_host):
+            if off[i + 1] == off[i]:
+                continue
+            if start == 0 and off[i + 1] - off[i] >= MIN_TOKENS:
+                fresh.append(i)
+            elif rest and rest[-1][1] == off[i]:
+                rest[-1][1] = off[i + 1]
+            else:
+                rest.append([off[i], off[i + 1]])
+        batch.plans["fresh"] = (fresh, rest) if fresh else None
+    return batch.plans["fresh"]
+
+
+def build_tiles(cu_seqlens: list, device, rows: int = TILE, sequences: Optional[list] = None) -> torch.Tensor:
     """[num_tiles, 4] int32 = (first token row, sequence length, q0, 0); most work first."""
     tiles = []
-    for s in range(len(cu_seqlens) - 1):
+    for s in sequences if sequences is not None else range(len(cu_seqlens) - 1):
         t0, n = cu_seqlens[s], cu_seqlens[s + 1] - cu_seqlens[s]
-        for q0 in range(0, n, TILE):
+        for q0 in range(0, n, rows):
             tiles.append((t0, n, q0, 0))
     tiles.sort(key=lambda t: -t[2])
     return torch.tensor(tiles, dtype=torch.int32, device=device)
 
 
-def prefill_attention(qkv, batch, hq, hkv, hd, *, sm_scale=None, quant_out=False):
+def prefill_attention(qkv, batch, hq, hkv, hd, *, sm_scale=None, quant_out=False, window=0, sinks=None, sequences=None, out=None):
+    """Rows of the fresh ``sequences`` (default: all) -> [T, hq * hd], a QTensor with ``quant_out`` (heads of 128); other rows of
+    the result are not written.  ``out`` supplies the result."""
     t = qkv.shape[0]
     scale = sm_scale if sm_scale is not None else 1.0 / math.sqrt(hd)
-    if batch.prefill_tiles is None:
-        batch.prefill_tiles = build_tiles(batch.cu_seqlens_host, qkv.device)
-    tiles = batch.prefill_tiles
-    wsp = workspace(qkv.device)
-    if quant_out:
-        oq = _alloc_q(t, hq * hd, qkv.device)
-        ob, o8, osc, ld = None, oq.data, oq.scale, t
-    else:
-        obt = torch.empty((t, hq * hd), dtype=torch.bfloat16, device=qkv.device)
-        ob, o8, osc, ld = obt, None, None, 0
-    rc = _lib.kernels().sllm_prefill_attention(_p(qkv), t, qkv.stride(0), _p(tiles), tiles.shape[0], hq, hkv, hd, scale,
-                                               _p(ob), _p(o8), _p(osc), ld, _p(wsp.status), _stream())
+    lib = _lib.kernels()
+    rows = lib.sllm_prefill_tile_rows(hq, hkv, hd)
+    key = ("prefill_tiles", rows, sequences is None)
+    tiles = batch.plans.get(key)
+    if tiles is None:
+        cu = batch.cu_seqlens_host if sequences is None else batch.row_off_host
+        tiles = batch.plans[key] = build_tiles(cu, qkv.device, rows, sequences)
+    if out is None:
+        out = _alloc_q(t, hq * hd, qkv.device) if quant_out else torch.empty((t, hq * hd), dtype=torch.bfloat16, device=qkv.device)
+    ob, o8, osc, ld = (None, out.data, out.scale, out.scale.stride(0)) if quant_out else (out, None, None, 0)
+    if _lib.audit_enabled():
+        _lib.record_dispatch("attention", "prefill_attention_kernel", rows=t, hq=hq, hkv=hkv, hd=hd, window=window,
+                             grid=[hq // 2 if rows == TILE and hd != 256 else hq, tiles.shape[0]])
+    rc = lib.sllm_prefill_attention(_p(qkv), t, qkv.stride(0), _p(tiles), tiles.shape[0], hq, hkv, hd, window, scale, _p(sinks),
+                                    _p(ob), _p(o8), _p(osc), ld, _p(workspace(qkv.device).status), _stream())
     _lib.check(rc, "prefill_attention")
-    return oq if quant_out else obt
+    return out
+
+
+def mixed_attention(q, qkv, kv, batch, part, hq, hkv, hd, *, sm_scale=None, quant_out=False, window=0, sinks=None):
+    """Attention of a batch of which ``part`` (of ``fresh_part``) are fresh prompts."""
+    fresh, rest = part
+    out = prefill_attention(qkv, batch, hq, hkv, hd, sm_scale=sm_scale, quant_out=quant_out, window=window, sinks=sinks, sequences=fresh)
+    for lo, hi in rest:
+        to = QTensor(out.data[lo:hi], out.scale[:, lo:hi]) if quant_out else out[lo:hi]
+        paged_attention(q[lo:hi], kv, batch.block_table, batch.seq_index[lo:hi], batch.kv_lens[lo:hi], hq, hkv, hd, window=window,
+                        sm_scale=sm_scale, max_kv=batch.max_kv, quant_out=quant_out, sinks=sinks, out=to)
+    return out
