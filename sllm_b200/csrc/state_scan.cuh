@@ -1,7 +1,7 @@
 // One step of a matrix-valued recurrent state, per head, S [dim keys, vdim values] in fp32:
 //   S <- diag(w) S - au (u^T S) + k v^T,   o = S^T r          (kRemoval: with the removal term, kPlain: without it)
 //   S <- g S;  S <- S + k (beta (v - S^T k))^T,   o = S^T q   (kGatedDelta: one decay g per head, beta v in place of v)
-// Columns of S (value channels) never meet, so heads are cut into column tiles.  A thread keeps 16 keys x 2 or 4 columns of S
+// Columns of S (value channels) never meet, so heads are cut into column tiles.  A thread keeps 16 keys x 1, 2 or 4 columns of S
 // in registers; kKL = 1 .. 32 lanes share a column.  All dot products of a token are taken from the OLD state in one sweep,
 //   o = (w r)^T S - (u^T S) (au^T r) + v k^T r,     o = g q^T S + (k^T q) (beta v - beta g k^T S)
 // so a token costs one shuffle reduction and no barrier.
@@ -172,7 +172,7 @@ __device__ __forceinline__ void state_token(float (&S)[kDrKeys][kC], const float
 
 template <int kKL, int kC, bool kStore>
 __device__ __forceinline__ void state_io(float (&S)[kDrKeys][kC], float* st, int dim, int vdim, int kl, int col) {
-  const bool whole = vdim % kC == 0;                 // col is a multiple of kC: its columns are one aligned access
+  const bool whole = kC > 1 && vdim % kC == 0;                 // col is a multiple of kC: its columns are one aligned access
 #pragma unroll
   for (int j = 0; j < kDrKeys / 4; ++j)
 #pragma unroll
@@ -183,7 +183,7 @@ __device__ __forceinline__ void state_io(float (&S)[kDrKeys][kC], float* st, int
       const bool in = key < dim && col < vdim;
       if constexpr (kStore) {
         if (in && whole) {
-          st_vec<kC>(ptr, x);
+          if constexpr (kC > 1) st_vec<kC>(ptr, x);
         } else if (in) {
 #pragma unroll
           for (int c = 0; c < kC; ++c)
@@ -193,7 +193,7 @@ __device__ __forceinline__ void state_io(float (&S)[kDrKeys][kC], float* st, int
 #pragma unroll
         for (int c = 0; c < kC; ++c) x[c] = 0.f;
         if (in && whole) {
-          ld_vec<kC>(ptr, x);
+          if constexpr (kC > 1) ld_vec<kC>(ptr, x);
         } else if (in) {
 #pragma unroll
           for (int c = 0; c < kC; ++c)
