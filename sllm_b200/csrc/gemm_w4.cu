@@ -146,7 +146,7 @@ gemm_w4_kernel(const __grid_constant__ CUtensorMap tm_x, const W4Params p) {
   uint8_t* stages = smem + 4 * kABufs * kW4ASlotBytes;
   W4Barriers* bars = reinterpret_cast<W4Barriers*>(stages + p.stages * kStageBytes);
   // one accumulator per issuer; the epilogue adds them up
-  constexpr uint32_t kTmemCols = kW4Issuers * BN < 32 ? 32 : kW4Issuers * BN;
+  constexpr uint32_t kTmemCols = BN == 96 ? 512 : kW4Issuers * BN;    // a power of two
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row_tile = blockIdx.x, split = blockIdx.z;
@@ -516,7 +516,7 @@ SLLM_EXPORT int sllm_gemm_w4_read_trace(long long* out1024) {
 
 // wtiles: the tiled resident weights (codes + scales, see the top of the file);
 // x: bf16 [total_tokens, k] with row stride ldx elements (columns k .. k_pad read as zero); y: bf16 [total_tokens, ldy].
-// fmt 0 = MXFP4, 1 = NVFP4.  bn in {16, 32, 64, 128}.  max_group_tokens bounds the tokens of any group
+// fmt 0 = MXFP4, 1 = NVFP4.  bn in {16, 32, 64, 96, 128}.  max_group_tokens bounds the tokens of any group
 // (dense: total_tokens).  Workspace: splits * total_tokens * n_valid floats and one counter per tile when splits > 1.
 static int gemm_w4_impl(const void* wtiles, const float* tensor_scale, const void* x, void* y,
                         const void* residual, const int* tok_off, const float* tok_scale, int fmt, int groups,
@@ -530,7 +530,7 @@ static int gemm_w4_impl(const void* wtiles, const float* tensor_scale, const voi
     return SLLM_ERR_INVALID_ARGUMENT;
   if (fmt != 0 && fmt != 1) return SLLM_ERR_INVALID_ARGUMENT;
   if (groups > 1 && !tok_off) return SLLM_ERR_INVALID_ARGUMENT;
-  if (bn != 16 && bn != 32 && bn != 64 && bn != 128) return SLLM_ERR_UNSUPPORTED_SHAPE;
+  if (bn != 16 && bn != 32 && bn != 64 && bn != 96 && bn != 128) return SLLM_ERR_UNSUPPORTED_SHAPE;
   if (reinterpret_cast<uintptr_t>(wtiles) & 15) return SLLM_ERR_ALIGNMENT;
   const int k_chunks = k_pad / kW4Chunk;
   if (splits < 1) splits = 1;
@@ -569,6 +569,7 @@ static int gemm_w4_impl(const void* wtiles, const float* tensor_scale, const voi
     SLLM_W4_CASE(16)
     SLLM_W4_CASE(32)
     SLLM_W4_CASE(64)
+    SLLM_W4_CASE(96)
     SLLM_W4_CASE(128)
   }
 #undef SLLM_W4_CASE
