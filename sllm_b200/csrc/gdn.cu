@@ -9,7 +9,7 @@
 //   beta    sigmoid(b) rounded to bf16;  decay = exp(-exp(A_log) * softplus(a + dt_bias))
 //   S      <- decay * S;  r = v - S k;  S <- S + beta * r k^T;  o = S q
 //   out     bf16(rmsnorm(bf16(o)) over dv, eps 1e-6) * norm_weight * silu(z)
-// One CTA per (sequence, value head), thread d owns row d of the state in registers for the whole sequence
+// Decode form: one CTA per (sequence, value head), thread d owns row d of the state in registers for the whole sequence
 // (the reference re-reads the state from memory for every token: linear_attention_kernel.hip.cpp:128; same
 // operation order here so that results agree with its fp32 oracle).
 #include "common.cuh"

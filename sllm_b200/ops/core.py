@@ -244,7 +244,7 @@ def linear(x, w: LinearWeight, residual: Optional[torch.Tensor] = None, act: Opt
     else:
         k_blocks = (w.in_features + 63) // 64
     y = torch.empty((m, n), dtype=torch.float32 if out_fp32 else torch.bfloat16, device=xd.device)
-    if w.kind != "fp8" and m > 1 and x.stride(0) != x.shape[1] and residual is not None:
+    if residual is not None and w.kind != "fp8" and m > 1 and x.stride(0) != x.shape[1]:
         raise ValueError("a product with a residual takes contiguous rows")
     # prompts: pairs of CTAs; it stores whole 16-byte units of bf16 rows, other widths and fp32 sums stay with the general kernel
     if m > 128 and n % 8 == 0 and not out_fp32 and (residual is None or (residual.is_contiguous() and residual.dtype == torch.bfloat16)):

@@ -28,13 +28,13 @@ def usable(q, batch, hd, window, sinks, qkv, quant_out: bool = False) -> bool:
     bit's difference moves them by a sixteenth: with a window or sinks they come from the pages."""
     if quant_out and (window or sinks is not None):
         return False
-    return _heads_fit(q, hd, qkv) and batch.cu_seqlens_host is not None and batch.max_seqlen >= MIN_TOKENS
+    return batch.cu_seqlens_host is not None and batch.max_seqlen >= MIN_TOKENS and _heads_fit(q, hd, qkv)
 
 
 def fresh_part(q, batch, hd, qkv) -> Optional[tuple]:
     """(sequences that take the kernel, [lo, hi) runs of the other rows) of a batch that mixes prompts with running requests, or
     None where no prompt of MIN_TOKENS starts in it."""
-    if not _heads_fit(q, hd, qkv) or batch.row_off_host is None or batch.starts_host is None or batch.row_off_host[-1] != q.shape[0]:
+    if batch.row_off_host is None or batch.starts_host is None:
         return None
     if "fresh" not in batch.plans:
         off, fresh, rest = batch.row_off_host, [], []
@@ -48,7 +48,8 @@ def fresh_part(q, batch, hd, qkv) -> Optional[tuple]:
             else:
                 rest.append([off[i], off[i + 1]])
         batch.plans["fresh"] = (fresh, rest) if fresh else None
-    return batch.plans["fresh"]
+    part = batch.plans["fresh"]
+    return part if part is not None and batch.row_off_host[-1] == q.shape[0] and _heads_fit(q, hd, qkv) else None
 
 
 def build_tiles(cu_seqlens: list, device, rows: int = TILE, sequences: Optional[list] = None) -> torch.Tensor:
