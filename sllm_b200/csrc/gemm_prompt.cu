@@ -70,6 +70,7 @@ struct GpParams {
   int epilogue;                             // 0 store, 1 add residual, 2 square of relu, 3 soft cap
   float act_arg;
   const float* alpha;                       // optional factor of the sums (bf16 operands)
+  int w_const;                              // no kernel writes w: its first tiles are requested ahead of the previous kernel's end
   const float *scale_x, *scale_w;           // [num_kb, ld]
   const __nv_bfloat16* residual;            // [m, ldy]
   int* status;
@@ -139,10 +140,11 @@ gemm_prompt_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
         auto load_x = [&](int s, int kb, int tm) {
           pair_tma_load_2d(smem + s * S::kStage, &tm_x, leader_addr(&sh->full[s]), kb * kElems, (tm * 2 + rank) * kGpRows);
         };
-        // the first stages' weights do not depend on the previous kernel
+        // the first stages' weights, which mostly do not depend on the previous kernel
         int tm, tn;
         gp_tile(p, pair, tm, tn);
         const int pre = min(p.num_kb, S::kStages);
+        if (!p.w_const) pdl_wait();
         for (int i = 0; i < pre; ++i) {
           if (rank == 0) mbar_expect_tx(&sh->full[i], 2 * S::kStage);
           load_w(i, i, tn);
@@ -412,10 +414,10 @@ using namespace sllm;
 
 // x [m, k] (row stride ldx elements), w [n, k] contiguous, y [m, n] bf16 (row stride ldy): bf16 operands, or with scale_x / scale_w
 // E4M3 and scales [ceil(k / 128), ld].  epilogue: 0 store, 1 add residual [m, ldy], 2 square of relu, 3 act_arg tanh(. / act_arg).
-// alpha: optional device scalar that multiplies the sums of bf16 operands.  bn: columns of a pair's tile, 64, 128 or 256.  n and ldy are multiples of 8, rows of x and w of 16 bytes.
+// alpha: optional device scalar that multiplies the sums of bf16 operands.  w_const: no kernel of the stream writes w.  bn: columns of a pair's tile, 64, 128 or 256.  n and ldy are multiples of 8, rows of x and w of 16 bytes.
 SLLM_EXPORT int sllm_gemm_prompt(const void* x, const void* w, void* y, const float* scale_x, const float* scale_w, const void* residual,
                                  int m, int n, int k, long long ldx, int ldy, int ld_sx, int ld_sw, int epilogue, float act_arg,
-                                 const float* alpha, int bn, int* status, void* stream) {
+                                 const float* alpha, int w_const, int bn, int* status, void* stream) {
   if (!x || !w || !y || m <= 0 || n <= 0 || k <= 0 || ldx < k || ldy < n || epilogue < 0 || epilogue > 3 || (epilogue == 1) != (residual != nullptr))
     return SLLM_ERR_INVALID_ARGUMENT;
   if (alpha && scale_x) return SLLM_ERR_UNSUPPORTED_SHAPE;
@@ -424,7 +426,7 @@ SLLM_EXPORT int sllm_gemm_prompt(const void* x, const void* w, void* y, const fl
   const bool scaled = scale_x != nullptr;
   GpParams p = {};
   p.m = m; p.n = n; p.num_kb = scaled ? (k + 127) / 128 : (k + 63) / 64;
-  p.ldy = ldy; p.ld_sx = ld_sx; p.ld_sw = ld_sw; p.epilogue = epilogue; p.act_arg = act_arg; p.alpha = alpha;
+  p.ldy = ldy; p.ld_sx = ld_sx; p.ld_sw = ld_sw; p.epilogue = epilogue; p.act_arg = act_arg; p.alpha = alpha; p.w_const = w_const;
   p.scale_x = scale_x; p.scale_w = scale_w; p.residual = static_cast<const __nv_bfloat16*>(residual); p.status = status;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   switch (bn) {

@@ -165,7 +165,7 @@ def _linear_prompt(x: torch.Tensor, w: LinearWeight, y: torch.Tensor, scale_x: O
                              grid=[min(148, 2 * ((m + 255) // 256) * ((n + bn - 1) // bn))])
     rc = _lib.kernels().sllm_gemm_prompt(_p(x), _p(w.w), _p(y), _p(scale_x), _p(w.scale_t) if scaled else None, _p(residual), m, n, k,
                                          x.stride(0), y.stride(0), scale_x.stride(0) if scaled else 0,
-                                         w.scale_t.stride(0) if scaled else 0, epilogue, act_arg, None, bn, _p(workspace(x.device).status),
+                                         w.scale_t.stride(0) if scaled else 0, epilogue, act_arg, None, 1, bn, _p(workspace(x.device).status),
                                          _stream())
     _lib.check(rc, "gemm_prompt")
 

@@ -270,7 +270,7 @@ def _linear_expanded(x: torch.Tensor, w: W4Weight, residual: Optional[torch.Tens
             _lib.record_dispatch("linear_w4", "gemm_prompt_kernel", fmt=w.fmt, tokens=t, n=rows, k=k, groups=1, grouped=False, bn=bn)
         res = None if residual is None else residual[:, r0:]
         rc = lib.sllm_gemm_prompt(_p(x), _p(dense), _p(y[:, r0:]), None, None, _p(res), t, rows, k, x.stride(0), w.n, 0, 0,
-                                  0 if residual is None else 1, 0.0, _p(w.tensor_scale), bn, status, _stream())
+                                  0 if residual is None else 1, 0.0, _p(w.tensor_scale), 0, bn, status, _stream())
         _lib.check(rc, "gemm_prompt")
     return y
 
