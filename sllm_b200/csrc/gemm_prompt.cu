@@ -22,8 +22,8 @@
 //   1500 x 2048 x 9216        129 ->   57                    106 ->   84
 //   5400 x 4096 x 14336       910 ->  420                    732 ->  557
 //   8192 x 28672 x 4096      3060 -> 1190 (1.62 PFLOP/s)    2497 -> 1620 (1.19 PFLOP/s)
-// bf16 at the last size moves 12.5 TB/s of operands out of L2, which is what holds it.  E4M3 spends about 2000 cycles a K block in
-// the promotion; reading the block's 128 x 256 sums out of tensor memory alone takes 560.
+// bf16 with 256 columns keeps the tensor pipe 96 % active (4096 x 14336 x 4096); narrower tiles are held by operands out of L2.  E4M3
+// spends about 2000 cycles a K block in the promotion (pipe 26 % active); reading 128 x 256 sums out of tensor memory alone takes 560.
 #include "pair_mma.cuh"
 #include "api.h"
 #include "tmap.h"

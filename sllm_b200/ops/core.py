@@ -140,7 +140,7 @@ def _gemm_plan(m: int, n: int, k_blocks: int):
 
 
 # Cycles of one 128-byte K block of a pair's tile by its columns (csrc/gemm_prompt.cu), measured with the machine full: bf16 is held
-# by L2 below 256 columns, E4M3 by the promotion of every block's sums
+# by L2 below 256 columns and by the tensor cores there, E4M3 by the promotion of every block's sums
 _PROMPT_BLOCK = {False: {64: 520, 128: 540, 256: 700}, True: {64: 830, 128: 1060, 256: 2050}}
 
 
