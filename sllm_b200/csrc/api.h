@@ -33,7 +33,7 @@ int sllm_gemm_allreduce(const void* a, const void* b, void* y, const float* scal
 /* gemm_prompt.cu */
 int sllm_gemm_prompt(const void* x, const void* w, void* y, const float* scale_x, const float* scale_w,
                      const void* residual, int m, int n, int k, long long ldx, int ldy, int ld_sx, int ld_sw,
-                     int epilogue, float act_arg, const float* alpha, int w_const, int bn, int* status,
+                     int epilogue, float act_arg, const float* alpha, int parts, int w_const, int bn, int* status,
                      void* stream);
 
 /* elementwise.cu */

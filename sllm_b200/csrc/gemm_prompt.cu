@@ -12,16 +12,22 @@
 //   warps 4 ..  epilogue, thread = output row: a group of four warps per 128 columns (64 for BN = 64)
 // Scaled: every K block has an accumulator of its own (two or four in turn), which the epilogue warps fold into fp32 registers with
 // scale_x[kb, m] scale_w[kb, n] while the next block is multiplied; fp32 pairs go through one instruction each.
+// bf16: the K blocks i, i + parts, i + 2 parts, .. form partial sum i, in an accumulator of its own, and the epilogue warps add the
+// partial sums in fp32 registers while the next one is multiplied.  Tensor memory rounds every addition towards zero, so that a
+// chain of K / 64 blocks in one accumulator is off by twice as much as two chains of half the length (2048 x 4096 x 14336 of one
+// sign: 7.0e-5 of the result against 3.0e-5, beyond the rounding to bf16).  The partial sums are those of the kernels that serve fewer
+// rows (two of gemm_tcgen05.cu's issuers, four of gemm_w4.cu's), so that results have the same bits on both sides of the line.
 // Tiles are visited in groups of eight columns of tiles, all rows within a group, so that what runs at one time shares its
 // operands in L2.  Tiles leave through shared memory: a warp stores its own 32 x 64 pieces and waits for no other.
 //
 // Measured (B200, one launch, m x n x k, us; before: the 128 x 128 tiles of gemm_tcgen05.cu):
 //                          bf16 before -> now             E4M3 before -> now
-//   130 x 4096 x 4096          38 ->   25                     38 ->   25
-//   527 x 6144 x 4096          70 ->   35                     58 ->   46
-//   1500 x 2048 x 9216        129 ->   57                    106 ->   84
-//   5400 x 4096 x 14336       910 ->  420                    732 ->  557
-//   8192 x 28672 x 4096      3060 -> 1190 (1.62 PFLOP/s)    2497 -> 1620 (1.19 PFLOP/s)
+//   130 x 4096 x 4096          38 ->   31                     38 ->   25
+//   527 x 6144 x 4096          70 ->   38                     58 ->   46
+//   1500 x 2048 x 9216        129 ->   61                    106 ->   83
+//   5400 x 4096 x 14336       910 ->  418                    732 ->  564
+//   8192 x 28672 x 4096      3060 -> 1197 (1.61 PFLOP/s)    2497 -> 1620 (1.19 PFLOP/s)
+// (bf16 in one chain per tile, which is less exact: 29, 36, 59, 408, 1195 us in the same run)
 // bf16 with 256 columns keeps the tensor pipe 96 % active (4096 x 14336 x 4096); narrower tiles are held by operands out of L2.  E4M3
 // spends about 2000 cycles a K block in the promotion (pipe 26 % active); reading 128 x 256 sums out of tensor memory alone takes 560.
 #include "pair_mma.cuh"
@@ -46,18 +52,20 @@ struct GpShape {
   static constexpr int kCols = BN / kGroups;               // columns per epilogue thread
   static constexpr int kThreads = 128 + 128 * kGroups;
   // 128 fp32 sums a thread need more than the 168 registers of 384 threads: the first four warps hand theirs over
-  static constexpr bool kMoveRegs = kScaled && kThreads == 384;
+  static constexpr bool kMoveRegs = kThreads == 384;
   static constexpr int kOutBytes = 4 * kGroups * 4096;     // 32 rows x 64 columns per epilogue warp
   static constexpr int kScaleBytes = kScaled ? kGpScaleRing * kGpScaleChunk * (kGpRows + BN) * 4 : 0;
-  static constexpr int kAcc = kScaled && BN < 256 ? 4 : 2; // accumulators
+  // accumulators: two of every partial sum that is under way; scaled: of K blocks in turn
+  static constexpr int kLive = kScaled || BN == 256 ? 1 : BN == 128 ? 2 : 4;
+  static constexpr int kAcc = kScaled && BN < 256 ? 4 : 2 * kLive;
   static constexpr uint32_t kTmem = kAcc * BN;
 };
 
 struct __align__(16) GpShared {
   uint64_t full[kGpMaxStages];              // first CTA's: the bytes of both
   uint64_t empty[kGpMaxStages];
-  uint64_t acc_full[4];
-  uint64_t acc_empty[4];                    // first CTA's: the epilogue warps of both
+  uint64_t acc_full[8];
+  uint64_t acc_empty[8];                    // first CTA's: the epilogue warps of both
   uint64_t scale_full[kGpScaleRing];
   uint64_t scale_empty[kGpScaleRing];
   uint32_t tmem_base;
@@ -66,6 +74,7 @@ struct __align__(16) GpShared {
 
 struct GpParams {
   int m, n, num_kb, tiles_m, tiles_n;
+  int parts;                                // partial sums of a tile (scaled: one chain, promoted block by block)
   int ldy, ld_sx, ld_sw;
   int epilogue;                             // 0 store, 1 add residual, 2 square of relu, 3 soft cap
   float act_arg;
@@ -86,6 +95,32 @@ __device__ __forceinline__ void gp_tile(const GpParams& p, int t, int& tm, int& 
   tm = r / wide;
   tn = g * kGpGroupN + r - tm * wide;
 }
+
+// The K blocks of a tile in the order that they are multiplied: kLive partial sums at a time, whose blocks come in turn (neighbours
+// along K share DRAM and L2 lines; 130 x 4096 x 4096 takes 32.8 us with one partial sum after the other, 30.7 with both at a time).
+template <int kLive>
+struct GpBlocks {
+  int kb = 0, part = 0, lo = 0, hi;                        // partial sums [lo, hi) are under way
+  __device__ __forceinline__ explicit GpBlocks(const GpParams& p) : hi(min(kLive, p.parts)) {}
+  __device__ __forceinline__ bool first() const { return kb == part; }
+  __device__ __forceinline__ bool last(const GpParams& p) const { return kb + p.parts >= p.num_kb; }
+  __device__ __forceinline__ void next(const GpParams& p) {
+    if constexpr (kLive == 1) {
+      kb += p.parts;
+      if (kb >= p.num_kb) kb = ++part;
+      return;
+    }
+    ++kb;
+    if (++part == hi) {
+      kb += p.parts - (hi - lo);
+      part = lo;
+    }
+    if (kb >= p.num_kb) {
+      kb = part = lo = hi;
+      hi = min(lo + kLive, p.parts);
+    }
+  }
+};
 
 template <int BN, bool kScaled>
 __global__ void __launch_bounds__(GpShape<BN, kScaled>::kThreads, 1)
@@ -145,16 +180,18 @@ gemm_prompt_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
         gp_tile(p, pair, tm, tn);
         const int pre = min(p.num_kb, S::kStages);
         if (!p.w_const) pdl_wait();
-        for (int i = 0; i < pre; ++i) {
+        GpBlocks<S::kLive> first(p);
+        for (int i = 0; i < pre; ++i, first.next(p)) {
           if (rank == 0) mbar_expect_tx(&sh->full[i], 2 * S::kStage);
-          load_w(i, i, tn);
+          load_w(i, first.kb, tn);
         }
         pdl_wait();
         int it = 0;                                        // K blocks over all tiles
         bool ok = true;
         for (int t = pair; ok && t < tiles; t += pairs) {
           gp_tile(p, t, tm, tn);
-          for (int kb = 0; kb < p.num_kb; ++kb, ++it) {
+          GpBlocks<S::kLive> b(p);
+          for (int i = 0; i < p.num_kb; ++i, ++it, b.next(p)) {
             const int s = it % S::kStages;
             if (it >= pre) {
               if (!mbar_wait(&sh->empty[s], ((it / S::kStages) & 1) ^ 1, abort_flag, p.status, SLLM_DEV_TIMEOUT_SMEM_EMPTY)) {
@@ -162,9 +199,9 @@ gemm_prompt_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
                 break;
               }
               if (rank == 0) mbar_expect_tx(&sh->full[s], 2 * S::kStage);
-              load_w(s, kb, tn);
+              load_w(s, b.kb, tn);
             }
-            load_x(s, kb, tm);
+            load_x(s, b.kb, tm);
           }
         }
         pdl_trigger();
@@ -179,30 +216,32 @@ gemm_prompt_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
     } else if (warp == 1) {
       if (rank == 0) {
         constexpr uint32_t idesc = make_idesc(kScaled ? kFmtE4M3 : kFmtBf16, 256, BN);
-        int it = 0, acc = 0;                               // acc: accumulators handed over so far
+        int it = 0, acc = 0;                               // acc: accumulators handed over by earlier tiles (scaled: blocks)
         bool ok = true;
         for (int t = pair; ok && t < tiles; t += pairs) {
-          for (int kb = 0; kb < p.num_kb; ++kb, ++it) {
-            const int s = it % S::kStages, buf = acc % S::kAcc;
+          GpBlocks<S::kLive> b(p);
+          for (int i = 0; i < p.num_kb; ++i, ++it, b.next(p)) {
+            const int s = it % S::kStages, use = kScaled ? acc : acc + b.part, buf = use % S::kAcc;
             ok = mbar_wait(&sh->full[s], (it / S::kStages) & 1, abort_flag, p.status, SLLM_DEV_TIMEOUT_TMA_FULL);
-            if (ok && (kScaled || kb == 0))
-              ok = mbar_wait(&sh->acc_empty[buf], ((acc / S::kAcc) & 1) ^ 1, abort_flag, p.status, SLLM_DEV_TIMEOUT_TMEM_EMPTY);
+            if (ok && (kScaled || b.first()))
+              ok = mbar_wait(&sh->acc_empty[buf], ((use / S::kAcc) & 1) ^ 1, abort_flag, p.status, SLLM_DEV_TIMEOUT_TMEM_EMPTY);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             tc_fence_after();
             const uint32_t a_addr = smem_u32(smem + s * S::kStage);
             const uint64_t ad = make_smem_desc_sw128(a_addr), bd = make_smem_desc_sw128(a_addr + S::kABytes);
-            const bool last = kScaled || kb == p.num_kb - 1;
+            const bool last = kScaled || b.last(p);
             if (elect_one()) {
 #pragma unroll
               for (int k = 0; k < 4; ++k)                  // 4 x 32 bytes of K
-                pair_umma<kScaled>(tmem_base + buf * BN, ad + 2 * k, bd + 2 * k, idesc, k > 0 || (!kScaled && kb > 0));
+                pair_umma<kScaled>(tmem_base + buf * BN, ad + 2 * k, bd + 2 * k, idesc, k > 0 || (!kScaled && !b.first()));
               pair_commit(&sh->empty[s]);
               if (last) pair_commit(&sh->acc_full[buf]);
             }
             __syncwarp();
-            acc += last;
+            if (kScaled) ++acc;
           }
+          if (!kScaled) acc += p.parts;
         }
       }
     } else if (kScaled) {
@@ -342,29 +381,35 @@ gemm_prompt_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
       }
     } else {
       const float alpha = p.alpha ? *p.alpha : 1.f;
-      for (int t = pair; ok && t < tiles; t += pairs, ++acc) {
+      for (int t = pair; ok && t < tiles; t += pairs) {
         int tm, tn;
         gp_tile(p, t, tm, tn);
-        ok = mbar_wait(&sh->acc_full[acc % S::kAcc], (acc / S::kAcc) & 1, abort_flag, p.status, SLLM_DEV_TIMEOUT_TMEM_FULL);
-        ok = __all_sync(0xffffffffu, ok);
+        float sum[S::kCols];
+#pragma unroll
+        for (int c = 0; c < S::kCols; ++c) sum[c] = 0.f;
+        for (int part = 0; part < p.parts; ++part, ++acc) {
+          ok = mbar_wait(&sh->acc_full[acc % S::kAcc], (acc / S::kAcc) & 1, abort_flag, p.status, SLLM_DEV_TIMEOUT_TMEM_FULL);
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          tc_fence_after();
+#pragma unroll
+          for (int c = 0; c < S::kCols / 32; ++c) {
+            uint32_t r[32];
+            tmem_ld32(lane_addr + (acc % S::kAcc) * BN + c * 32, r);
+            tmem_wait_regs(r);
+#pragma unroll
+            for (int j = 0; j < 32; ++j) sum[c * 32 + j] += __uint_as_float(r[j]);
+          }
+          tc_fence_before();                               // all of it is in registers
+          __syncwarp();
+          if (lane == 0) mbar_arrive_remote(empty_addr + 8 * (acc % S::kAcc));
+        }
         if (!ok) break;
-        tc_fence_after();
 #pragma unroll
         for (int c = 0; c < S::kCols / 64; ++c) {
           float v[64];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            uint32_t r[16];
-            tmem_ld16(lane_addr + (acc % S::kAcc) * BN + c * 64 + i * 16, r);
-            tmem_wait_regs(r);
-#pragma unroll
-            for (int j = 0; j < 16; ++j) v[i * 16 + j] = __uint_as_float(r[j]) * alpha;
-          }
-          if (c == S::kCols / 64 - 1) {                    // all of it is in registers
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_remote(empty_addr + 8 * (acc % S::kAcc));
-          }
+          for (int i = 0; i < 64; ++i) v[i] = sum[c * 64 + i] * alpha;
           emit(v, (tm * 2 + rank) * kGpRows + q * 32, tn * BN + grp * S::kCols + c * 64);
         }
       }
@@ -414,18 +459,22 @@ using namespace sllm;
 
 // x [m, k] (row stride ldx elements), w [n, k] contiguous, y [m, n] bf16 (row stride ldy): bf16 operands, or with scale_x / scale_w
 // E4M3 and scales [ceil(k / 128), ld].  epilogue: 0 store, 1 add residual [m, ldy], 2 square of relu, 3 act_arg tanh(. / act_arg).
-// alpha: optional device scalar that multiplies the sums of bf16 operands.  w_const: no kernel of the stream writes w.  bn: columns of a pair's tile, 64, 128 or 256.  n and ldy are multiples of 8, rows of x and w of 16 bytes.
+// alpha: optional device scalar that multiplies the sums of bf16 operands.  parts: partial sums of bf16 operands, 1 to 4 (K blocks of 64
+// taken in turn).  w_const: no kernel of the stream writes w.  bn: columns of a pair's tile, 64, 128 or 256.  n and ldy are multiples
+// of 8, rows of x and w of 16 bytes.
 SLLM_EXPORT int sllm_gemm_prompt(const void* x, const void* w, void* y, const float* scale_x, const float* scale_w, const void* residual,
                                  int m, int n, int k, long long ldx, int ldy, int ld_sx, int ld_sw, int epilogue, float act_arg,
-                                 const float* alpha, int w_const, int bn, int* status, void* stream) {
+                                 const float* alpha, int parts, int w_const, int bn, int* status, void* stream) {
   if (!x || !w || !y || m <= 0 || n <= 0 || k <= 0 || ldx < k || ldy < n || epilogue < 0 || epilogue > 3 || (epilogue == 1) != (residual != nullptr))
     return SLLM_ERR_INVALID_ARGUMENT;
-  if (alpha && scale_x) return SLLM_ERR_UNSUPPORTED_SHAPE;
+  if (parts < 1 || parts > 4) return SLLM_ERR_INVALID_ARGUMENT;
+  if (scale_x && (alpha || parts != 1)) return SLLM_ERR_UNSUPPORTED_SHAPE;
   if (!scale_x != !scale_w || (scale_x && (ld_sx < m || ld_sw < n))) return SLLM_ERR_INVALID_ARGUMENT;
   if ((n & 7) || (ldy & 7) || (reinterpret_cast<uintptr_t>(residual) & 15)) return SLLM_ERR_ALIGNMENT;
   const bool scaled = scale_x != nullptr;
   GpParams p = {};
   p.m = m; p.n = n; p.num_kb = scaled ? (k + 127) / 128 : (k + 63) / 64;
+  p.parts = parts < p.num_kb ? parts : p.num_kb;
   p.ldy = ldy; p.ld_sx = ld_sx; p.ld_sw = ld_sw; p.epilogue = epilogue; p.act_arg = act_arg; p.alpha = alpha; p.w_const = w_const;
   p.scale_x = scale_x; p.scale_w = scale_w; p.residual = static_cast<const __nv_bfloat16*>(residual); p.status = status;
   cudaStream_t st = static_cast<cudaStream_t>(stream);

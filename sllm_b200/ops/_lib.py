@@ -167,7 +167,7 @@ _KERNEL_SIGNATURES = {
     "sllm_gemm_workspace_floats": (L, [I, I, I, I]),
     "sllm_gemm": (I, [P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, I, P, L, P, I, P, P]),
     "sllm_gemm_act": (I, [P, P, P, I, I, I, I, I, I, I, F, I, I, I, I, P, L, P, I, P, P]),
-    "sllm_gemm_prompt": (I, [P, P, P, P, P, P, I, I, I, L, I, I, I, I, F, P, I, I, P, P]),
+    "sllm_gemm_prompt": (I, [P, P, P, P, P, P, I, I, I, L, I, I, I, I, F, P, I, I, I, P, P]),
     "sllm_w4_expand": (I, [P, P, I, I, I, I, I, I, P]),
     "sllm_gemm_simt": (I, [P, P, P, P, I, I, I, I, I, I, I, F, I, I, P]),
     "sllm_group_norm": (I, [P, P]),

@@ -144,6 +144,9 @@ def _gemm_plan(m: int, n: int, k_blocks: int):
 _PROMPT_BLOCK = {False: {64: 520, 128: 540, 256: 700}, True: {64: 830, 128: 1060, 256: 2050}}
 
 
+_GEMM_PARTS = 2            # partial sums of a bf16 product (two issuers of the 128-column tiles in csrc/gemm_tcgen05.cu)
+
+
 def _prompt_tile(m: int, n: int, scaled: bool) -> int:
     """Columns of a tile of the prompt product: the fewest cycles over the waves of 74 CTA pairs, 256 rows a pair.  Narrow tiles
     spread few rows over more pairs (130 x 4096 x 4096: 25 us with 64 columns, 31 with 256), wide ones reuse their operands
@@ -165,8 +168,8 @@ def _linear_prompt(x: torch.Tensor, w: LinearWeight, y: torch.Tensor, scale_x: O
                              grid=[min(148, 2 * ((m + 255) // 256) * ((n + bn - 1) // bn))])
     rc = _lib.kernels().sllm_gemm_prompt(_p(x), _p(w.w), _p(y), _p(scale_x), _p(w.scale_t) if scaled else None, _p(residual), m, n, k,
                                          x.stride(0), y.stride(0), scale_x.stride(0) if scaled else 0,
-                                         w.scale_t.stride(0) if scaled else 0, epilogue, act_arg, None, 1, bn, _p(workspace(x.device).status),
-                                         _stream())
+                                         w.scale_t.stride(0) if scaled else 0, epilogue, act_arg, None, 1 if scaled else _GEMM_PARTS, 1, bn,
+                                         _p(workspace(x.device).status), _stream())
     _lib.check(rc, "gemm_prompt")
 
 

@@ -243,6 +243,7 @@ def _bn_for(tokens: int) -> int:
     return 16 if tokens <= 16 else 32 if tokens <= 32 else 64 if tokens <= 64 else 96 if tokens <= 96 else 128
 
 
+PARTS = 4                      # partial sums of a product (four issuers in csrc/gemm_w4.cu)
 EXPAND_ELEMENTS = 1 << 27      # of an expanded weight at a time (256 MB)
 
 
@@ -270,7 +271,7 @@ def _linear_expanded(x: torch.Tensor, w: W4Weight, residual: Optional[torch.Tens
             _lib.record_dispatch("linear_w4", "gemm_prompt_kernel", fmt=w.fmt, tokens=t, n=rows, k=k, groups=1, grouped=False, bn=bn)
         res = None if residual is None else residual[:, r0:]
         rc = lib.sllm_gemm_prompt(_p(x), _p(dense), _p(y[:, r0:]), None, None, _p(res), t, rows, k, x.stride(0), w.n, 0, 0,
-                                  0 if residual is None else 1, 0.0, _p(w.tensor_scale), 0, bn, status, _stream())
+                                  0 if residual is None else 1, 0.0, _p(w.tensor_scale), PARTS, 0, bn, status, _stream())
         _lib.check(rc, "gemm_prompt")
     return y
 

@@ -40,6 +40,18 @@ def test_tiles(monkeypatch, scaled, m, n, k, bn):
     assert ops.device_status(torch.device(DEV, 0)) == 0
 
 
+@pytest.mark.parametrize("m,n,k", [(129, 8, 64), (300, 264, 128), (257, 520, 192), (385, 1032, 1040), (1030, 136, 4096), (2600, 8200, 320)])
+@pytest.mark.parametrize("bn", [64, 128, 256])
+def test_partial_sums_are_those_of_the_general_product(monkeypatch, m, n, k, bn):
+    """Two chains of K blocks, added in fp32: the same bits as the kernel that serves fewer rows."""
+    monkeypatch.setattr(core, "_prompt_tile", lambda *a: bn)
+    x, w, _, _, r = _operands(m, n, k, False, m + k)
+    for res in (None, r):
+        want = torch.empty(m, n, dtype=torch.bfloat16, device=DEV)
+        core.gemm_raw(x, w.w, want, residual=res, transpose_out=False, bn=128, splits=1, stages=5)
+        assert torch.equal(ops.linear(x, w, res), want)
+
+
 def test_many_tiles_per_pair():
     """More tiles than pairs: accumulators, stages and scale chunks wrap around across tiles."""
     for scaled in (False, True):

@@ -28,6 +28,18 @@ def test_expanded_products(monkeypatch, fmt, t, n, k):
     assert ops.device_status(torch.device(DEV, 0)) == 0
 
 
+@pytest.mark.parametrize("fmt", ["mxfp4", "nvfp4"])
+@pytest.mark.parametrize("t,n,k", [(129, 136, 64), (260, 640, 200), (300, 1032, 384), (1076, 4096, 4096)])
+def test_expanded_products_have_the_bits_of_packed_ones(fmt, t, n, k):
+    """Four chains of K blocks, added in fp32, on both sides."""
+    g = torch.Generator(device=DEV).manual_seed(t)
+    weight = W4Weight.quantize_device(fmt, torch.randn(n, k, generator=g, device=DEV) * 0.05)
+    x = torch.randn(t, k, generator=g, device=DEV).bfloat16()
+    r = torch.randn(t, n, generator=g, device=DEV).bfloat16()
+    for res in (None, r):
+        assert torch.equal(linear_w4(x, weight, residual=res), linear_w4(x, weight, residual=res, splits=1))
+
+
 @pytest.mark.parametrize("counts", [[0, 0, 300], [17, 0, 64, 65, 1, 128, 0, 129], [3] * 70, [0] * 40 + [200, 5]])
 def test_token_tiles_of_experts(counts):
     g = torch.Generator(device=DEV).manual_seed(len(counts))
