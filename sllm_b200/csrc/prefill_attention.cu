@@ -4,15 +4,18 @@
 // rotated) and start at position 0, so K and V are read from that tensor with TMA instead of from the paged cache.  Optional sliding
 // window (key tiles outside it are not visited) and attention sinks.
 //
-// What bounds it: exponentials (16 a clock and SM) and products take about as long, 1024 cycles each for 128 queries x 128 keys x 128
-// channels, so neither may wait for the other.  A CTA carries two items, 128-row query tiles that share their keys and values: two
+// What bounds it: exponentials (16 a clock and SM) take 1024 cycles for 128 queries x 128 keys, products 512 (S) and 1024 (P V, twice)
+// with 128 channels, so neither may wait for the other.  A CTA carries two items, 128-row query tiles that share their keys and values: two
 // heads of a group (or, with one query head per kv head, two neighbouring tiles of one head).  While one item's softmax runs, the
 // tensor cores work on the other.  Heads of 256 channels fill the tensor memory with one item; its next scores are computed ahead.
 //
 //   warp 0      TMA producer: Q once, then K and V tiles through rings of two stages
 //   warp 1      TMEM owner; issues S = Q K^T and O += P V of all items
 //   warps 4 ..  softmax, four warps per item, thread = query row: the row's scores are read once into registers, P goes back to
-//               tensor memory in place of S (bf16, the A operand of the second product), O stays in tensor memory
+//               tensor memory in place of S as the A operand of the second product, O stays in tensor memory
+// P enters its product as two bf16 values, hi = bf16(p) and lo = bf16(p - hi), 16 significant bits that are multiplied one after the other;
+// the row's sum takes p itself.  Results are as far from 64 bits as their rounding to bf16 takes them (2-norm 0.00166), as with the fp32
+// probabilities of attention.cu; one bf16 value gives 0.0021 (4000 tokens, heads of 128: 0.00204 with the maximum of every tile).
 // With E4M3 results (kStrict) a row keeps O in registers, o <- o alpha + P V of the tile with the maximum of every tile, and reads its
 // scores twice: the next product quantises, where a last bit's difference becomes a sixteenth of a value, and this order is the one
 // that FP8 models have been run and compared with.
@@ -20,10 +23,11 @@
 // as exact, and sums hold 2^8 times larger values with ease.
 //
 // Measured (B200, us; before: one item per CTA whose scores, softmax and products followed one another, or the pages' rows one by one):
-//   8192 tokens, 32 + 2 x 8 heads x 128              2324 ->  542 (1.02 PFLOP/s), E4M3 results 1344
-//   2048 + 1098 + 1623 + 674 tokens, the same heads   431 ->  127,                E4M3 results  234
-//   2048 + 782 tokens, 16 + 2 x 4 heads x 256        3285 ->   83
-//   1000 + 536 + 823 tokens, 64 + 2 x 8 heads x 64    880 ->   81, with a window of 128 66
+//   8192 tokens, 32 + 2 x 8 heads x 128              2324 ->  662 (0.83 PFLOP/s), E4M3 results 1373
+//   2048 + 1098 + 1623 + 674 tokens, the same heads   431 ->  145,                E4M3 results  257
+//   2048 + 782 tokens, 16 + 2 x 4 heads x 256        3285 ->   90
+//   1000 + 536 + 823 tokens, 64 + 2 x 8 heads x 64    880 ->   87, with a window of 128 69
+// (P as one bf16 value: 532, 127, 79, 78 and 66 in the same run)
 // Replaces the reference's scalar prefill kernels (causal_attention_kernel.hip.cpp:388-495).
 #include "pair_mma.cuh"
 #include "api.h"
@@ -41,11 +45,10 @@ struct PfShape {
   static constexpr int kQBytes = kChunks * kPfTile * 128;  // of an item; chunks of [rows x 64 channels], 128-byte swizzle
   static constexpr int kKvBytes = kChunks * kKeys * 128;   // of a K or V tile
   static constexpr int kThreads = 128 + 128 * kItems;
-  // tensor memory: two score tiles (of the items, or of the even and odd tiles of one item), O of the items, then P where there is
-  // room for it (heads of 128 channels keep it in the first columns of its scores, which the next product into them overwrites
-  // after the one that reads P)
+  // tensor memory: two score tiles (of the items, or of the even and odd tiles of one item), then O of the items.  P takes the place of
+  // its scores: of 32 keys the upper halves of the values in 16 columns and the lower ones in the next 16.  The next product into
+  // these columns is issued after the one that reads P.
   static constexpr uint32_t kTmemO = 2 * kKeys;
-  static constexpr uint32_t kTmemP = HD == 128 ? 0 : kTmemO + kItems * HD, kPStride = HD == 128 ? kKeys : kKeys / 2;
   static constexpr size_t kSmem = kItems * kQBytes + 4 * kKvBytes + 256 + 1024;
 };
 
@@ -106,10 +109,29 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
       : "memory");
 }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// 2^x; kNormal: a subnormal result becomes zero.
+template <bool kNormal>
 __device__ __forceinline__ float pf_ex2(float x) {
   float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  if constexpr (kNormal) asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  else asm("ex2.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+// P of 32 keys from their scores: 2^(s scale - m), as a sum of two 16-bit values (16 significant bits), and the sums of P.
+template <bool kNormal>
+__device__ __forceinline__ void pf_probabilities(const uint32_t (&s)[32], float scale, float m, uint32_t (&hi)[16], uint32_t (&lo)[16],
+                                                 float (&sum)[4]) {
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const float p0 = pf_ex2<kNormal>(fmaf(__uint_as_float(s[2 * i]), scale, -m));
+    const float p1 = pf_ex2<kNormal>(fmaf(__uint_as_float(s[2 * i + 1]), scale, -m));
+    __nv_bfloat162 h = __floats2bfloat162_rn(p0, p1);
+    hi[i] = *reinterpret_cast<const uint32_t*>(&h);
+    h = __floats2bfloat162_rn(p0 - __uint_as_float(hi[i] << 16), p1 - __uint_as_float(hi[i] & 0xffff0000u));
+    lo[i] = *reinterpret_cast<const uint32_t*>(&h);
+    sum[2 * (i & 1)] += p0;
+    sum[2 * (i & 1) + 1] += p1;
+  }
 }
 
 // The rows of kStrict: heads of 128 channels, O in registers.  Scores are read for the maximum and again for the exponentials; P(32 keys)
@@ -320,9 +342,12 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
         const uint32_t va = v_addr + (j & 1) * S::kKvBytes;
         if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < kKeys / 16; ++k)             // 16 keys, 8 columns of P
-            umma_f16_ts(tmem_base + S::kTmemO + i * HD, tmem_base + S::kTmemP + b * S::kPStride + k * 8,
-                        make_smem_desc_sw128_mn(va + k * 16 * 128, kKeys * 128), idesc_pv, (!kStrict && j > 0) || k > 0);
+          for (int k = 0; k < kKeys / 16; ++k) {           // 16 keys, 8 columns of P
+            const uint64_t vd = make_smem_desc_sw128_mn(va + k * 16 * 128, kKeys * 128);
+            const uint32_t o = tmem_base + S::kTmemO + i * HD, pa = tmem_base + b * kKeys + (kStrict ? k * 8 : k / 2 * 32 + (k & 1) * 8);
+            umma_f16_ts(o, pa, vd, idesc_pv, (!kStrict && j > 0) || k > 0);
+            if (!kStrict) umma_f16_ts(o, pa + 16, vd, idesc_pv, 1);
+          }
           tc_commit(&bars->o_full[i]);
           if (i == kItems - 1) tc_commit(&bars->v_empty[j & 1]);
         }
@@ -370,7 +395,6 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
     for (int j = 0; j < nt; ++j) {
       const int b = kItems == 2 ? item : j & 1;
       const uint32_t ph = (kItems == 2 ? j : j >> 1) & 1, s_addr = lane_addr + b * kKeys;
-      const uint32_t p_addr = lane_addr + S::kTmemP + b * S::kPStride;
       ok = __all_sync(0xffffffffu, mbar_wait(&bars->s_full[b], ph, abort_flag, p.status, SLLM_DEV_TIMEOUT_TMEM_FULL));
       if (!ok) break;
       tc_fence_after();
@@ -380,11 +404,18 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
 #pragma unroll
       for (int c = 0; c < kKeys / 32; ++c) tmem_wait_regs(sr[c]);
       const int k0 = first + j * kKeys;
-      if (k0 + kKeys - 1 > qt || (p.window > 0 && k0 <= qt + kPfTile - 1 - p.window)) {
-        const int hi = qpos - k0, lo = p.window > 0 ? hi - p.window + 1 : 0;   // keys [lo, hi] of the tile are visible
+      const bool edge = k0 + kKeys - 1 > qt || (p.window > 0 && k0 <= qt + kPfTile - 1 - p.window);
+      const int hi = edge ? qpos - k0 : kKeys, lo = edge && p.window > 0 ? qpos - k0 - p.window + 1 : 0;   // keys [lo, hi] are visible
+      float mn[4] = {INFINITY, INFINITY, INFINITY, INFINITY};                // of visible keys
+      if (edge) {
 #pragma unroll
-        for (int i = 0; i < kKeys; ++i)
+        for (int i = 0; i < kKeys; ++i) {
           if (i > hi || i < lo) sr[i >> 5][i & 31] = 0xff800000u;
+          else mn[i & 3] = fminf(mn[i & 3], __uint_as_float(sr[i >> 5][i & 31]));
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < kKeys; ++i) mn[i & 3] = fminf(mn[i & 3], __uint_as_float(sr[i >> 5][i & 31]));
       }
       float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
@@ -394,7 +425,7 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
       if (m == -INFINITY) {
         m = m_new;                                         // nothing but zeros in O and l
       } else if (m_new > m + 8.f) {
-        alpha = pf_ex2(m - m_new);
+        alpha = pf_ex2<false>(m - m_new);
         l *= alpha;
         m = m_new;
       }
@@ -414,21 +445,29 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
       }
       const float m_use = m == -INFINITY ? 0.f : m;
       float sum[4] = {0.f, 0.f, 0.f, 0.f};
+      if (__any_sync(0xffffffffu, fmaf(fminf(fminf(mn[0], mn[1]), fminf(mn[2], mn[3])), p.scale_log2, -m_use) < -126.f)) {
+        // subnormal probabilities: the exact exponential takes three instructions more, so it has a way of its own that reads the
+        // scores again (8192 tokens, 32 heads x 128: 715 us with it throughout)
+#pragma unroll 1
+        for (int c = 0; c < kKeys / 32; ++c) {
+          uint32_t v[32], h[16], e[16];
+          tmem_ld32(s_addr + c * 32, v);
+          tmem_wait_regs(v);
 #pragma unroll
-      for (int c = 0; c < kKeys / 64; ++c) {               // 64 keys = 32 columns
-        uint32_t w[32];
-#pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          const int k = c * 64 + 2 * i;
-          const float p0 = pf_ex2(fmaf(__uint_as_float(sr[k >> 5][k & 31]), p.scale_log2, -m_use));
-          const float p1 = pf_ex2(fmaf(__uint_as_float(sr[k >> 5][(k & 31) + 1]), p.scale_log2, -m_use));
-          const __nv_bfloat162 h = __floats2bfloat162_rn(p0, p1);
-          w[i] = *reinterpret_cast<const uint32_t*>(&h);
-          // the sum uses the rounded values, so the normaliser matches what the product multiplies
-          sum[2 * (i & 1)] += __uint_as_float(w[i] << 16);
-          sum[2 * (i & 1) + 1] += __uint_as_float(w[i] & 0xffff0000u);
+          for (int i = 0; i < 32; ++i)
+            if (c * 32 + i > hi || c * 32 + i < lo) v[i] = 0xff800000u;
+          pf_probabilities<false>(v, p.scale_log2, m_use, h, e, sum);
+          tmem_st16(s_addr + c * 32, h);
+          tmem_st16(s_addr + c * 32 + 16, e);
         }
-        tmem_st32(p_addr + c * 32, w);
+      } else {
+#pragma unroll
+        for (int c = 0; c < kKeys / 32; ++c) {
+          uint32_t h[16], e[16];
+          pf_probabilities<true>(sr[c], p.scale_log2, m_use, h, e, sum);
+          tmem_st16(s_addr + c * 32, h);
+          tmem_st16(s_addr + c * 32 + 16, e);
+        }
       }
       l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
       tmem_wait_st();
@@ -446,7 +485,7 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
       tc_fence_after();
     }
     if (ok) {
-      if (p.sinks && l > 0.f) l += pf_ex2(fmaf(p.sinks[head], 1.4426950408889634f, -m));
+      if (p.sinks && l > 0.f) l += pf_ex2<false>(fmaf(p.sinks[head], 1.4426950408889634f, -m));
       const float inv = l > 0.f ? 1.f / l : 0.f;
       const bool live = qpos < seq_len;
       const size_t row = static_cast<size_t>(tok0 + qpos), base = (row * p.hq + head) * HD;
