@@ -23,7 +23,7 @@
 // as exact, and sums hold 2^8 times larger values with ease.
 //
 // Measured (B200, us; before: one item per CTA whose scores, softmax and products followed one another, or the pages' rows one by one):
-//   8192 tokens, 32 + 2 x 8 heads x 128              2324 ->  662 (0.83 PFLOP/s), E4M3 results 1373
+//   8192 tokens, 32 + 2 x 8 heads x 128              2324 ->  671 (0.82 PFLOP/s), E4M3 results 1355
 //   2048 + 1098 + 1623 + 674 tokens, the same heads   431 ->  145,                E4M3 results  257
 //   2048 + 782 tokens, 16 + 2 x 4 heads x 256        3285 ->   90
 //   1000 + 536 + 823 tokens, 64 + 2 x 8 heads x 64    880 ->   87, with a window of 128 69
@@ -361,6 +361,7 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
       bool ok = wait(&bars->q_full, 0, SLLM_DEV_TIMEOUT_TMA_FULL) && wait(&bars->k_full[0], 0, SLLM_DEV_TIMEOUT_TMA_FULL);
       if (ok)
         for (int i = 0; i < kItems; ++i) issue_s(i, 0);
+      const int own = seq_len - first - (nt - 1) * kKeys;  // keys of the last tile that are the sequence's (or more)
       for (int j = 0; ok && j < nt; ++j) {
         const bool more = j + 1 < nt;
         if (kItems == 1 && more) {                         // the next scores run under this tile's softmax
@@ -369,6 +370,16 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
           issue_s(0, j + 1);
         }
         ok = wait(&bars->v_full[j & 1], (j >> 1) & 1, SLLM_DEV_TIMEOUT_TMA_FULL);
+        // Rows behind the sequence are another request's: their P is zero, but zero times an infinity of theirs would not be.
+        // (Only the last tile has any; its stage is not filled again.)
+        if (!more && own < kKeys) {
+          uint8_t* v = v_s + (j & 1) * S::kKvBytes;
+          for (int c = 0; c < S::kChunks; ++c)
+            for (int e = (c * kKeys + own) * 8 + lane; e < (c + 1) * kKeys * 8; e += 32)       // 16-byte units
+              *reinterpret_cast<uint4*>(v + e * 16) = make_uint4(0, 0, 0, 0);
+          fence_proxy_async_smem();
+          __syncwarp();
+        }
         for (int i = 0; ok && i < kItems; ++i) {
           ok = kItems == 2 ? wait(&bars->p_ready[i], j & 1, SLLM_DEV_TIMEOUT_TMEM_EMPTY)
                            : wait(&bars->p_ready[j & 1], (j >> 1) & 1, SLLM_DEV_TIMEOUT_TMEM_EMPTY);

@@ -106,3 +106,47 @@ def test_subnormal_probabilities_stay(hd):
     want = ((row + 1) / 2).floor() / (row / 2 + 1).floor() * 2.0 ** -10
     # a subnormal of 2^-130 has 19 bits, its exponent an error of 130 2^-23; then one rounding
     assert ((got - want).abs() <= want * (2.0 ** -8 + 2.0 ** -14)).all()
+
+
+@pytest.mark.parametrize("hd", [64, 128, 256])
+@pytest.mark.parametrize("hq,hkv", [(2, 2), (4, 1)])
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+@pytest.mark.parametrize("window", [0, 100])
+def test_a_request_does_not_reach_its_neighbours(hd, hq, hkv, value, window):
+    """Rows of a request whose values are not finite lie behind another request's in the last tile of keys."""
+    lens = [129, 140, 257, 1, 383]
+    g = torch.Generator(device=DEV).manual_seed(hd + hq)
+    qkv = torch.randn(sum(lens), (hq + 2 * hkv) * hd, generator=g, device=DEV).bfloat16()
+    b = make_prefill_batch([[0] * n for n in lens], torch.zeros((len(lens), 1), dtype=torch.int32, device=DEV), DEV)
+    broken = qkv.clone()
+    broken[129:129 + 140, hq * hd:] = value                # keys and values of the second and the fourth
+    broken[129 + 140 + 257, hq * hd:] = value
+    keep = torch.cat([torch.full((n,), i not in (1, 3), device=DEV) for i, n in enumerate(lens)])
+    for quant in (False, True) if hd == 128 and not window else (False,):
+        want, got = (prefill.prefill_attention(x, b, hq, hkv, hd, window=window, quant_out=quant) for x in (qkv, broken))
+        if quant:
+            assert torch.equal(got.data[keep], want.data[keep]) and torch.equal(got.scale[:, keep], want.scale[:, keep])
+        else:
+            assert want.isfinite().all() and torch.equal(got[keep], want[keep])
+
+
+def test_a_request_does_not_reach_its_neighbours_in_a_mixed_batch():
+    hq, hkv, hd, page = 8, 2, 128, 16
+    starts, counts = [0, 77, 0, 40, 0], [300, 1, 140, 33, 150]
+    g = torch.Generator(device=DEV).manual_seed(4)
+    t, blocks = sum(counts), 320 // page
+    qkv = torch.randn(t, (hq + 2 * hkv) * hd, generator=g, device=DEV).bfloat16()
+    results = []
+    for bad in (False, True):
+        kv = KVLayer(*(torch.ones(5 * blocks, hkv, page, hd, device=DEV).bfloat16() for _ in range(2)), None, None, False, page)
+        table = torch.arange(5 * blocks, dtype=torch.int32, device=DEV).view(5, blocks)
+        b = make_prefill_batch([[0] * c for c in counts], table, DEV, starts)
+        x = qkv.clone()
+        if bad:
+            x[300, (hq + hkv) * hd:] = float("inf")          # the second request's only row
+            x[441:474, (hq + hkv) * hd:] = float("nan")      # the fourth's
+        q = ops.rope_kv_append(x, b.positions, b.seq_index, b.block_table, kv, hq, hkv, hd, 1e4)
+        assert prefill.fresh_part(q, b, hd, x)[0] == [0, 2, 4]
+        results.append(ops.attention(q, kv, b, hq, hkv, hd, qkv=x))
+    keep = torch.cat([torch.full((c,), i not in (1, 3), device=DEV) for i, c in enumerate(counts)])
+    assert torch.equal(results[0][keep], results[1][keep])
