@@ -467,6 +467,7 @@ SLLM_EXPORT int sllm_gemm_prompt(const void* x, const void* w, void* y, const fl
                                  const float* alpha, int parts, int w_const, int bn, int* status, void* stream) {
   if (!x || !w || !y || m <= 0 || n <= 0 || k <= 0 || ldx < k || ldy < n || epilogue < 0 || epilogue > 3 || (epilogue == 1) != (residual != nullptr))
     return SLLM_ERR_INVALID_ARGUMENT;
+  if (epilogue == 3 && !(act_arg > 0.f)) return SLLM_ERR_INVALID_ARGUMENT;
   if (parts < 1 || parts > 4) return SLLM_ERR_INVALID_ARGUMENT;
   if (scale_x && (alpha || parts != 1)) return SLLM_ERR_UNSUPPORTED_SHAPE;
   if (!scale_x != !scale_w || (scale_x && (ld_sx < m || ld_sw < n))) return SLLM_ERR_INVALID_ARGUMENT;

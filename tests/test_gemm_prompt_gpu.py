@@ -69,3 +69,11 @@ def test_activations_and_strided_rows():
     wide = torch.zeros(300, 512, device=DEV, dtype=torch.bfloat16)
     wide[:, 8:264] = x
     _close(ops.linear(wide[:, 8:264], w), want, xf, wf)
+
+
+@pytest.mark.parametrize("m", [1, 128, 129, 300])
+@pytest.mark.parametrize("cap", [0.0, -1.0, float("nan")])
+def test_a_soft_cap_that_is_not_positive_is_refused(m, cap):
+    x, w, _, _, _ = _operands(m, 64, 64, False, 1)
+    with pytest.raises(ops.KernelError):
+        ops.linear(x, w, act="softcap", act_arg=cap)
