@@ -469,7 +469,7 @@ SLLM_EXPORT int sllm_gdn_recurrent(const void* qkv, const void* z, const void* b
   return e == cudaSuccess ? SLLM_OK : SLLM_ERR_CUDA;
 }
 
-// The prompt form (three launches).  tokens = rows of qkv; scratch: fp32, at least
+// The prompt form (three launches).  tokens = rows of qkv, which starts at a multiple of 4 bytes; scratch: fp32, at least
 // tokens * (2 * qk_heads * 128 + 2 * v_heads + v_heads * 128) elements.
 SLLM_EXPORT int sllm_gdn_recurrent_prompt(const void* qkv, const void* z, const void* b, const void* a, const float* a_log,
                                           const void* dt_bias, const float* norm_w, float* state, void* out,
@@ -480,6 +480,7 @@ SLLM_EXPORT int sllm_gdn_recurrent_prompt(const void* qkv, const void* z, const 
       sequences <= 0 || tokens <= 0 || qk_heads <= 0 || v_heads <= 0 || (v_heads % qk_heads))
     return SLLM_ERR_INVALID_ARGUMENT;
   if (head_dim != kGdnHeadDim) return SLLM_ERR_UNSUPPORTED_SHAPE;
+  if (reinterpret_cast<uintptr_t>(qkv) & 3) return SLLM_ERR_ALIGNMENT;        // the scan copies two values at a time
   const long long nq = static_cast<long long>(tokens) * qk_heads * kGdnHeadDim;
   const long long ng = static_cast<long long>(tokens) * v_heads * 2;
   const long long no = static_cast<long long>(tokens) * v_heads * kGdnHeadDim;

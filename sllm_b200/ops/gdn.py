@@ -124,6 +124,8 @@ def recurrent(qkv, z, b, a, a_log, dt_bias, norm_w, state, row_off, slots, qk_he
     if t >= PROMPT_FORM_MIN_ROWS_PER_SEQUENCE * slots.numel() and prompt_form_enabled():
         # prompts: the state-independent work (q / k normalisation, gates, output norm) runs in parallel over the
         # tokens, the scan itself carries no reduction (three launches; a decode step keeps the fused kernel)
+        if qkv.data_ptr() % 4:
+            qkv = qkv.clone()                       # the scan copies pairs of channels
         n = t * (2 * qk_heads * hd + 2 * v_heads + v_heads * hd)
         scratch = torch.empty((n,), dtype=torch.float32, device=qkv.device)
         rc = _k().sllm_gdn_recurrent_prompt(_p(qkv), _p(z), _p(b), _p(a), _p(a_log), _p(dt_bias), _p(norm_w), _p(state), _p(out),
