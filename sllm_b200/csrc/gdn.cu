@@ -66,7 +66,8 @@ gdn_conv_rows_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* _
   constexpr int kHist = kTaps - 1;
   const int c = (blockIdx.x * 256 + threadIdx.x) * 2;
   if (c >= width) return;
-  const int first = blockIdx.y * kConvRun, last = min(tokens, first + kConvRun);
+  const int run = blockIdx.y * kConvRun, last = min(tokens, run + kConvRun);
+  const int first = max(run, row_off[0]);              // rows ahead of the first sequence are nobody's
   int s = 0;
   for (int hi = sequences - 1; s < hi;) {              // the last sequence that starts at or before the first row
     const int mid = (s + hi + 1) >> 1;

@@ -27,6 +27,22 @@ def test_conv_rows(taps, counts, width):
     assert torch.equal(got_st.cpu(), st)
 
 
+@pytest.mark.parametrize("ahead", [1, 31, 32, 70])
+def test_conv_rows_ahead_of_the_first_sequence(ahead):
+    """Offsets that do not start at row 0: the rows ahead belong to no sequence and no history is read for them."""
+    counts, width, taps = [40, 33], 130, 4
+    g = torch.Generator().manual_seed(ahead)
+    t = ahead + sum(counts)
+    off = torch.tensor([ahead] + [ahead + int(c) for c in np.cumsum(counts)], dtype=torch.int32)
+    slots = torch.tensor([1, 0], dtype=torch.int32)
+    x, w = torch.randn(t, width, generator=g).bfloat16(), (torch.randn(width, taps, generator=g) * 0.3).bfloat16()
+    st = torch.randn(2, taps - 1, width, generator=g).bfloat16()
+    got_st = st.to(DEV)
+    want = gdn.conv_silu(x, w, st, off, slots)[ahead:].float()
+    got = gdn.conv_silu(x.to(DEV), w.to(DEV), got_st, off.to(DEV), slots.to(DEV))[ahead:].float().cpu()
+    assert (got - want).abs().max() <= 2.0 ** -7 * want.abs().max() and torch.equal(got_st.cpu(), st)
+
+
 def test_recurrence_from_an_odd_element():
     """A contiguous qkv that starts between two 4-byte words: copied by the op, refused by the kernel's entry before any launch."""
     g = torch.Generator().manual_seed(3)
