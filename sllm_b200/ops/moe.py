@@ -189,9 +189,9 @@ def shared_add(a: torch.Tensor, b: torch.Tensor, gate: torch.Tensor) -> torch.Te
 
 
 def expert_mlp(x: torch.Tensor, tok_off: torch.Tensor, perm_src: torch.Tensor, perm_w: torch.Tensor, gate_up: W4Weight,
-               down: W4Weight, act: str, row_ptr: Optional[torch.Tensor] = None) -> Optional[torch.Tensor]:
+               down: W4Weight, act: str, row_ptr: Optional[torch.Tensor] = None, experts: int = 0) -> Optional[torch.Tensor]:
     """The gated MLP of the local experts over the routed rows (grouped by expert: `tok_off`), routing weights applied:
-    y_perm [T*k, d], or None when `row_ptr` scatters the rows (see `linear_w4`).
+    y_perm [T*k, d], or None when `row_ptr` scatters the rows (see `linear_w4`).  `experts`: those of all ranks (0: all are local).
 
     W4A16 (default): gather rows -> grouped gate_up GEMM -> SiLU*up -> grouped down GEMM, bf16 activations.
     W4A4 (`ops.w4.set_w4a4`): the quantiser reads the routed rows in place (no gather), both GEMMs run on the
@@ -201,7 +201,7 @@ def expert_mlp(x: torch.Tensor, tok_off: torch.Tensor, perm_src: torch.Tensor, p
     from . import w4 as W
     t = x.shape[0]
     # 4-bit activations serve the decode regime; with more than 32 routed rows per expert on average (a prompt) the
-    # rows are compute bound and keep bf16 activations on the W4A16 kernel, whose token tiles are 128 wide
+    # rows are compute bound and keep bf16 activations on the W4A16 kernel, whose token tiles hold up to 128
     if W.w4a4_enabled() and x.dtype == torch.bfloat16 and perm_src.numel() <= W.W4A4_MAX_DENSE_ROWS * gate_up.groups:
         rows = perm_src.numel()
         n_rows = tok_off[-1:] if x.is_cuda else None
@@ -216,16 +216,16 @@ def expert_mlp(x: torch.Tensor, tok_off: torch.Tensor, perm_src: torch.Tensor, p
             y = torch.cat([y, y.new_zeros((perm_src.numel() - y.shape[0], y.shape[1]))])
         return y
     xp = gather(x, perm_src, tok_off)
-    a = core.gated_act(linear_w4(xp, gate_up, tok_off=tok_off, max_group_tokens=t), act)
-    return linear_w4(a, down, tok_off=tok_off, tok_scale=perm_w, max_group_tokens=t, row_ptr=row_ptr)
+    a = core.gated_act(linear_w4(xp, gate_up, tok_off=tok_off, max_group_tokens=t, experts=experts), act)
+    return linear_w4(a, down, tok_off=tok_off, tok_scale=perm_w, max_group_tokens=t, row_ptr=row_ptr, experts=experts)
 
 
 def experts_forward(x: torch.Tensor, idx: torch.Tensor, w: torch.Tensor, gate_up: W4Weight, down: W4Weight, act: str,
-                    e_lo: int, e_hi: int):
-    """Runs the local experts [e_lo, e_hi) on the tokens routed to them.  Returns (y_perm [T*k, d] with the routing
-    weights applied, perm_dst [T, k])."""
+                    e_lo: int, e_hi: int, experts: int = 0):
+    """Runs the local experts [e_lo, e_hi) (of `experts` on all ranks) on the tokens routed to them.  Returns (y_perm [T*k, d]
+    with the routing weights applied, perm_dst [T, k])."""
     tok_off, perm_src, perm_dst, perm_w = permute(idx, w, e_lo, e_hi)
-    return expert_mlp(x, tok_off, perm_src, perm_w, gate_up, down, act), perm_dst
+    return expert_mlp(x, tok_off, perm_src, perm_w, gate_up, down, act, experts=experts), perm_dst
 
 
 # ------------------------------------------------------------------------------------------ experts with dense weights

@@ -243,6 +243,14 @@ def _bn_for(tokens: int) -> int:
     return 16 if tokens <= 16 else 32 if tokens <= 32 else 64 if tokens <= 64 else 96 if tokens <= 96 else 128
 
 
+def _group_tile(rows: int, most: int, experts: int) -> int:
+    """Token columns of a grouped product: a tile that holds the mean of the groups with a quarter to spare, so that few groups convert
+    their weights twice (62 rows for each of 128 experts, a call of two layers: 6.8 ms in tiles of 64, 5.2 of 96, 6.3 of 128).  ``rows``
+    are those of all ``experts`` of the layer, also where a rank holds some.  The spread is not known here: 2 rows for each of 128
+    experts take 7 % less in tiles of 16 than of 32 (a call of 64 tokens), all of 1024 rows on 16 of them 41 % more (one product)."""
+    return _bn_for(min(most, 5 * rows // (4 * experts)))
+
+
 PARTS = 4                      # partial sums of a product (four issuers in csrc/gemm_w4.cu)
 EXPAND_ELEMENTS = 1 << 27      # of an expanded weight at a time (256 MB)
 
@@ -278,9 +286,10 @@ def _linear_expanded(x: torch.Tensor, w: W4Weight, residual: Optional[torch.Tens
 
 def linear_w4(x: torch.Tensor, w: W4Weight, residual: Optional[torch.Tensor] = None, tok_off: Optional[torch.Tensor] = None,
               tok_scale: Optional[torch.Tensor] = None, max_group_tokens: Optional[int] = None, splits: int = 0,
-              row_ptr: Optional[torch.Tensor] = None) -> Optional[torch.Tensor]:
+              row_ptr: Optional[torch.Tensor] = None, experts: int = 0) -> Optional[torch.Tensor]:
     """y[t, :] = x[t, :] @ W_g(t)^T (* tok_scale[t]) (+ residual).  Dense when tok_off is None (groups must be 1);
-    grouped otherwise: tokens of group g are rows tok_off[g] .. tok_off[g + 1] of x."""
+    grouped otherwise: tokens of group g are rows tok_off[g] .. tok_off[g + 1] of x.  ``experts``: among how many the t rows were
+    spread, where the weight holds one rank's share of them (0: the weight's groups)."""
     if isinstance(x, Fp4Act):
         if x.k != w.k or x.fmt != w.fmt:
             raise ValueError("quantised activations do not match the weight's width or format")
@@ -319,9 +328,7 @@ def linear_w4(x: torch.Tensor, w: W4Weight, residual: Optional[torch.Tensor] = N
     x = x.contiguous() if x.stride(1) != 1 or x.stride(0) % 8 else x
     y = torch.empty((t, w.n), dtype=torch.bfloat16, device=x.device)
     mgt = max_group_tokens or t
-    # grouped: a tile that holds the mean of the groups with a quarter to spare, so that few groups convert their weights twice
-    # (62 rows for each of 128 experts, a call of two layers: 6.8 ms in tiles of 64, 5.2 of 96, 6.3 of 128)
-    bn = _bn_for(mgt if tok_off is None else min(mgt, 5 * t // (4 * w.groups)))
+    bn = _bn_for(mgt) if tok_off is None else _group_tile(t, mgt, experts or w.groups)
     k_chunks = w.k_pad // 128
     if splits <= 0:
         ctas = (w.n_rows // 128) * (w.groups if tok_off is None else max(1, min(w.groups, t))) * ((min(mgt, t) + bn - 1) // bn)

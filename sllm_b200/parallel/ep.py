@@ -33,7 +33,7 @@ class NoEP:
 
     def experts_combine(self, x, idx, rw, gate_up, down, act: str, e_lo: int, e_hi: int, residual):
         """Routed experts of this rank on `x` and the sum over all ranks (+ residual): the MoE block after routing."""
-        yp, perm_dst = M.experts_forward(x, idx, rw, gate_up, down, act, e_lo, e_hi)
+        yp, perm_dst = M.experts_forward(x, idx, rw, gate_up, down, act, e_lo, e_hi, (e_hi - e_lo) * self.size)
         return self.combine(yp, perm_dst, residual)
 
 
@@ -126,7 +126,7 @@ class FusedEP(NcclEP):
         rc = lib.sllm_moe_owner_plan(*peers, _p(perm_dst), t, k, self.d, tpr, _p(self.owner_epoch), _p(row_ptr), _stream())
         _lib.check(rc, "moe_owner_plan")
         # the down projection stores every routed row (route weight applied) into its owner's slot, on whatever GPU
-        M.expert_mlp(x, tok_off, perm_src, perm_w, gate_up, down, act, row_ptr=row_ptr)
+        M.expert_mlp(x, tok_off, perm_src, perm_w, gate_up, down, act, row_ptr=row_ptr, experts=(e_hi - e_lo) * self.size)
         y = torch.empty((t, self.d), dtype=torch.bfloat16, device=x.device)
         rc = lib.sllm_moe_owner_combine(*peers, k, _p(residual), _p(y), t, self.d, tpr, self.rows_per_block,
                                         _p(self.owner_epoch), _p(self.owner_counter), _p(workspace(x.device).status), _stream())
