@@ -91,8 +91,26 @@ def mixed_attention(q, qkv, kv, batch, part, hq, hkv, hd, *, sm_scale=None, quan
     """Attention of a batch of which ``part`` (of ``fresh_part``) are fresh prompts."""
     fresh, rest = part
     out = prefill_attention(qkv, batch, hq, hkv, hd, sm_scale=sm_scale, quant_out=quant_out, window=window, sinks=sinks, sequences=fresh)
-    for lo, hi in rest:
-        to = QTensor(out.data[lo:hi], out.scale[:, lo:hi]) if quant_out else out[lo:hi]
-        paged_attention(q[lo:hi], kv, batch.block_table, batch.seq_index[lo:hi], batch.kv_lens[lo:hi], hq, hkv, hd, window=window,
-                        sm_scale=sm_scale, max_kv=batch.max_kv, quant_out=quant_out, sinks=sinks, out=to)
+    if not rest:
+        return out
+
+    def paged(rows, seq_index, kv_lens, to=None):
+        return paged_attention(rows, kv, batch.block_table, seq_index, kv_lens, hq, hkv, hd, window=window, sm_scale=sm_scale,
+                               max_kv=batch.max_kv, quant_out=quant_out, sinks=sinks, out=to)
+
+    if len(rest) == 1:
+        lo, hi = rest[0]
+        paged(q[lo:hi], batch.seq_index[lo:hi], batch.kv_lens[lo:hi],
+              QTensor(out.data[lo:hi], out.scale[:, lo:hi]) if quant_out else out[lo:hi])
+        return out
+    # rows in several runs: gathered, so that there is one launch however they lie
+    if "paged_rows" not in batch.plans:
+        idx = torch.tensor([r for lo, hi in rest for r in range(lo, hi)], device=q.device)
+        batch.plans["paged_rows"] = (idx, batch.seq_index[idx], batch.kv_lens[idx])
+    idx, seq_index, kv_lens = batch.plans["paged_rows"]
+    got = paged(q[idx], seq_index, kv_lens)
+    if quant_out:
+        out.data[idx], out.scale[:, idx] = got.data, got.scale
+    else:
+        out[idx] = got
     return out

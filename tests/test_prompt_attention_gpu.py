@@ -6,7 +6,7 @@ import torch
 
 from sllm_b200 import ops
 from sllm_b200.engine.batch import make_prefill_batch
-from sllm_b200.ops import prefill
+from sllm_b200.ops import _lib, prefill
 from sllm_b200.ops.core import KVLayer
 
 pytestmark = pytest.mark.gpu
@@ -150,3 +150,26 @@ def test_a_request_does_not_reach_its_neighbours_in_a_mixed_batch():
         results.append(ops.attention(q, kv, b, hq, hkv, hd, qkv=x))
     keep = torch.cat([torch.full((c,), i not in (1, 3), device=DEV) for i, c in enumerate(counts)])
     assert torch.equal(results[0][keep], results[1][keep])
+
+
+def test_rows_between_prompts_take_one_launch():
+    """Prompts and other rows in turn: the others are gathered for the pages."""
+    hq, hkv, hd, page = 8, 2, 128, 16
+    starts, counts = [5, 0, 77, 0, 40, 0, 3, 0, 9], [1, 300, 1, 129, 20, 150, 2, 128, 1]
+    g = torch.Generator(device=DEV).manual_seed(6)
+    t, blocks = sum(counts), 320 // page
+    kv = KVLayer(*(torch.randn(9 * blocks, hkv, page, hd, generator=g, device=DEV).bfloat16() for _ in range(2)), None, None, False, page)
+    table = torch.arange(9 * blocks, dtype=torch.int32, device=DEV).view(9, blocks)
+    b = make_prefill_batch([[0] * c for c in counts], table, DEV, starts)
+    qkv = torch.randn(t, (hq + 2 * hkv) * hd, generator=g, device=DEV).bfloat16()
+    q = ops.rope_kv_append(qkv, b.positions, b.seq_index, b.block_table, kv, hq, hkv, hd, 1e4)
+    want = ops.paged_attention(q, kv, table, b.seq_index, b.kv_lens, hq, hkv, hd, max_kv=b.max_kv).double()
+    for _ in range(2):                                  # the second call (another layer) uses the same plans
+        _lib.dispatch_records(clear=True)
+        _lib.audit(True)
+        try:
+            got = ops.attention(q, kv, b, hq, hkv, hd, qkv=qkv)
+        finally:
+            _lib.audit(False)
+        assert [e["kernel"] for e in _lib.dispatch_records(clear=True)] == ["prefill_attention_kernel", "paged_attention_kernel"]
+        _close(got, want, 2)
