@@ -23,8 +23,8 @@
 // as exact, and sums hold 2^8 times larger values with ease.
 //
 // Measured (B200, us; before: one item per CTA whose scores, softmax and products followed one another, or the pages' rows one by one):
-//   8192 tokens, 32 + 2 x 8 heads x 128              2324 ->  671 (0.82 PFLOP/s), E4M3 results 1355
-//   2048 + 1098 + 1623 + 674 tokens, the same heads   431 ->  145,                E4M3 results  257
+//   8192 tokens, 32 + 2 x 8 heads x 128              2324 ->  671 (0.82 PFLOP/s), E4M3 results 1260
+//   2048 + 1098 + 1623 + 674 tokens, the same heads   431 ->  147,                E4M3 results  241
 //   2048 + 782 tokens, 16 + 2 x 4 heads x 256        3285 ->   90
 //   1000 + 536 + 823 tokens, 64 + 2 x 8 heads x 64    880 ->   87, with a window of 128 69
 // (P as one bf16 value: 532, 127, 79, 78 and 66 in the same run)
@@ -134,10 +134,10 @@ __device__ __forceinline__ void pf_probabilities(const uint32_t (&s)[32], float 
   }
 }
 
-// The rows of kStrict: heads of 128 channels, O in registers.  Scores are read for the maximum and again for the exponentials; P(32 keys)
+// The rows of kStrict: heads of 128 channels without window and sinks, O in registers.  Scores are read for the maximum and again for the exponentials; P(32 keys)
 // overwrites score columns that have been read.
 __device__ __forceinline__ void strict_rows(const PrefillParams& p, PrefillBarriers* bars, uint32_t lane_addr, uint32_t o_addr, int item, int head,
-                                            int qt, int qpos, int first, int nt, int tok0, int seq_len, volatile int* abort_flag) {
+                                            int qt, int qpos, int nt, int tok0, int seq_len, volatile int* abort_flag) {
   constexpr int HD = 128, kKeys = 128;
   const uint32_t s_addr = lane_addr + item * kKeys;
   float o[HD];
@@ -149,9 +149,7 @@ __device__ __forceinline__ void strict_rows(const PrefillParams& p, PrefillBarri
     ok = __all_sync(0xffffffffu, mbar_wait(&bars->s_full[item], j & 1, abort_flag, p.status, SLLM_DEV_TIMEOUT_TMEM_FULL));
     if (!ok) break;
     tc_fence_after();
-    const int k0 = first + j * kKeys;
-    const bool edge = k0 + kKeys - 1 > qt || (p.window > 0 && k0 <= qt + kPfTile - 1 - p.window);
-    const int hi = edge ? qpos - k0 : kKeys, lo = edge && p.window > 0 ? qpos - k0 - p.window + 1 : 0;   // keys [lo, hi] are visible
+    const int k0 = j * kKeys, hi = k0 + kKeys - 1 > qt ? qpos - k0 : kKeys;     // keys up to hi are visible
     float tmax = -INFINITY;
 #pragma unroll
     for (int c = 0; c < 4; ++c) {
@@ -161,7 +159,7 @@ __device__ __forceinline__ void strict_rows(const PrefillParams& p, PrefillBarri
 #pragma unroll
       for (int i = 0; i < 32; ++i) {
         const float x = __uint_as_float(v[i]);
-        tmax = fmaxf(tmax, c * 32 + i > hi || c * 32 + i < lo ? -INFINITY : x);
+        tmax = fmaxf(tmax, c * 32 + i > hi ? -INFINITY : x);
       }
     }
     const float m_new = fmaxf(m, tmax * p.scale_log2);
@@ -177,8 +175,8 @@ __device__ __forceinline__ void strict_rows(const PrefillParams& p, PrefillBarri
       for (int i = 0; i < 16; ++i) {
         const int k = c * 32 + 2 * i;
         float p0 = exp2f(__uint_as_float(v[2 * i]) * p.scale_log2 - m_use), p1 = exp2f(__uint_as_float(v[2 * i + 1]) * p.scale_log2 - m_use);
-        if (k > hi || k < lo) p0 = 0.f;
-        if (k + 1 > hi || k + 1 < lo) p1 = 0.f;
+        if (k > hi) p0 = 0.f;
+        if (k + 1 > hi) p1 = 0.f;
         const __nv_bfloat162 h = __floats2bfloat162_rn(p0, p1);
         psum += __bfloat162float(h.x) + __bfloat162float(h.y);
         w[i] = *reinterpret_cast<const uint32_t*>(&h);
@@ -203,7 +201,6 @@ __device__ __forceinline__ void strict_rows(const PrefillParams& p, PrefillBarri
     }
     tc_fence_before();
   }
-  if (ok && p.sinks && l > 0.f) l += exp2f(p.sinks[head] * 1.4426950408889634f - m);
   if (ok && qpos < seq_len) {
     const float inv = l > 0.f ? 1.f / l : 0.f;
     const size_t row = static_cast<size_t>(tok0 + qpos), base = (row * p.hq + head) * HD;
@@ -401,7 +398,7 @@ prefill_attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
     float m = -INFINITY, l = 0.f;
     bool ok = true;
     if constexpr (kStrict) {
-      strict_rows(p, bars, lane_addr, o_addr, item, head, qt, qpos, first, nt, tok0, seq_len, abort_flag);
+      strict_rows(p, bars, lane_addr, o_addr, item, head, qt, qpos, nt, tok0, seq_len, abort_flag);
     } else {
     for (int j = 0; j < nt; ++j) {
       const int b = kItems == 2 ? item : j & 1;
@@ -561,12 +558,13 @@ SLLM_EXPORT int sllm_prefill_tile_rows(int hq, int hkv, int hd) {
 
 // tiles: device int32 [num_tiles][4] = {first token row of the sequence, sequence length, q0, 0}, q0 in steps of
 // sllm_prefill_tile_rows, ordered by the caller (most keys first).  qkv row stride is qkv_ld elements.  window: 0 or the number of
-// positions that a row sees; sinks: optional [hq].
+// positions that a row sees; sinks: optional [hq].  E4M3 results (out_fp8, out_scale): heads of 128 without window and sinks.
 SLLM_EXPORT int sllm_prefill_attention(const void* qkv, int total_tokens, int qkv_ld, const int* tiles, int num_tiles,
                                        int hq, int hkv, int hd, int window, float sm_scale, const float* sinks, void* out_bf16,
                                        void* out_fp8, float* out_scale, int ld_scale, int* status, void* stream) {
   if (!qkv || !tiles || num_tiles <= 0 || hq <= 0 || hkv <= 0 || hq % hkv || window < 0) return SLLM_ERR_INVALID_ARGUMENT;
-  if ((hd != 64 && hd != 128 && hd != 256) || (out_fp8 && hd != 128)) return SLLM_ERR_UNSUPPORTED_SHAPE;
+  if ((hd != 64 && hd != 128 && hd != 256) || (out_fp8 && (hd != 128 || window || sinks)))
+    return SLLM_ERR_UNSUPPORTED_SHAPE;
   if (!out_bf16 && !(out_fp8 && out_scale)) return SLLM_ERR_INVALID_ARGUMENT;
   if (num_tiles > 65535) return SLLM_ERR_LIMIT;
   if ((reinterpret_cast<uintptr_t>(out_bf16) | reinterpret_cast<uintptr_t>(out_fp8)) & 15) return SLLM_ERR_ALIGNMENT;

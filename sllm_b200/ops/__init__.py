@@ -12,7 +12,6 @@ def attention(q, kv, batch, hq, hkv, hd, *, window=0, quant_out=False, sm_scale=
         return prefill.prefill_attention(qkv, batch, hq, hkv, hd, sm_scale=sm_scale, quant_out=quant_out, window=window, sinks=sinks)
     part = None if quant_out else prefill.fresh_part(q, batch, hd, qkv)      # (E4M3 results of mixed batches: from the pages)
     if part is not None:
-        return prefill.mixed_attention(q, qkv, kv, batch, part, hq, hkv, hd, sm_scale=sm_scale, quant_out=quant_out, window=window,
-                                       sinks=sinks)
+        return prefill.mixed_attention(q, qkv, kv, batch, part, hq, hkv, hd, sm_scale=sm_scale, window=window, sinks=sinks)
     return paged_attention(q, kv, batch.block_table, batch.seq_index, batch.kv_lens, hq, hkv, hd, window=window,
                            sm_scale=sm_scale, max_kv=batch.max_kv, quant_out=quant_out, sinks=sinks)

@@ -12,7 +12,7 @@ from typing import Optional
 import torch
 
 from . import _lib
-from .core import QTensor, _alloc_q, _p, _stream, paged_attention, workspace
+from .core import _alloc_q, _p, _stream, paged_attention, workspace
 
 MIN_TOKENS = 128
 TILE = 128
@@ -63,9 +63,9 @@ def build_tiles(cu_seqlens: list, device, rows: int = TILE, sequences: Optional[
     return torch.tensor(tiles, dtype=torch.int32, device=device)
 
 
-def prefill_attention(qkv, batch, hq, hkv, hd, *, sm_scale=None, quant_out=False, window=0, sinks=None, sequences=None, out=None):
-    """Rows of the fresh ``sequences`` (default: all) -> [T, hq * hd], a QTensor with ``quant_out`` (heads of 128); other rows of
-    the result are not written.  ``out`` supplies the result."""
+def prefill_attention(qkv, batch, hq, hkv, hd, *, sm_scale=None, quant_out=False, window=0, sinks=None, sequences=None):
+    """Rows of the fresh ``sequences`` (default: all) -> [T, hq * hd], a QTensor with ``quant_out`` (heads of 128 without window and
+    sinks); other rows of the result are not written."""
     t = qkv.shape[0]
     scale = sm_scale if sm_scale is not None else 1.0 / math.sqrt(hd)
     lib = _lib.kernels()
@@ -75,8 +75,7 @@ def prefill_attention(qkv, batch, hq, hkv, hd, *, sm_scale=None, quant_out=False
     if tiles is None:
         cu = batch.cu_seqlens_host if sequences is None else batch.row_off_host
         tiles = batch.plans[key] = build_tiles(cu, qkv.device, rows, sequences)
-    if out is None:
-        out = _alloc_q(t, hq * hd, qkv.device) if quant_out else torch.empty((t, hq * hd), dtype=torch.bfloat16, device=qkv.device)
+    out = _alloc_q(t, hq * hd, qkv.device) if quant_out else torch.empty((t, hq * hd), dtype=torch.bfloat16, device=qkv.device)
     ob, o8, osc, ld = (None, out.data, out.scale, out.scale.stride(0)) if quant_out else (out, None, None, 0)
     if _lib.audit_enabled():
         _lib.record_dispatch("attention", "prefill_attention_kernel", rows=t, hq=hq, hkv=hkv, hd=hd, window=window,
@@ -87,30 +86,25 @@ def prefill_attention(qkv, batch, hq, hkv, hd, *, sm_scale=None, quant_out=False
     return out
 
 
-def mixed_attention(q, qkv, kv, batch, part, hq, hkv, hd, *, sm_scale=None, quant_out=False, window=0, sinks=None):
-    """Attention of a batch of which ``part`` (of ``fresh_part``) are fresh prompts."""
+def mixed_attention(q, qkv, kv, batch, part, hq, hkv, hd, *, sm_scale=None, window=0, sinks=None):
+    """Attention of a batch of which ``part`` (of ``fresh_part``) are fresh prompts; bf16 results."""
     fresh, rest = part
-    out = prefill_attention(qkv, batch, hq, hkv, hd, sm_scale=sm_scale, quant_out=quant_out, window=window, sinks=sinks, sequences=fresh)
+    out = prefill_attention(qkv, batch, hq, hkv, hd, sm_scale=sm_scale, window=window, sinks=sinks, sequences=fresh)
     if not rest:
         return out
 
     def paged(rows, seq_index, kv_lens, to=None):
         return paged_attention(rows, kv, batch.block_table, seq_index, kv_lens, hq, hkv, hd, window=window, sm_scale=sm_scale,
-                               max_kv=batch.max_kv, quant_out=quant_out, sinks=sinks, out=to)
+                               max_kv=batch.max_kv, sinks=sinks, out=to)
 
     if len(rest) == 1:
         lo, hi = rest[0]
-        paged(q[lo:hi], batch.seq_index[lo:hi], batch.kv_lens[lo:hi],
-              QTensor(out.data[lo:hi], out.scale[:, lo:hi]) if quant_out else out[lo:hi])
+        paged(q[lo:hi], batch.seq_index[lo:hi], batch.kv_lens[lo:hi], out[lo:hi])
         return out
     # rows in several runs: gathered, so that there is one launch however they lie
     if "paged_rows" not in batch.plans:
         idx = torch.tensor([r for lo, hi in rest for r in range(lo, hi)], device=q.device)
         batch.plans["paged_rows"] = (idx, batch.seq_index[idx], batch.kv_lens[idx])
     idx, seq_index, kv_lens = batch.plans["paged_rows"]
-    got = paged(q[idx], seq_index, kv_lens)
-    if quant_out:
-        out.data[idx], out.scale[:, idx] = got.data, got.scale
-    else:
-        out[idx] = got
+    out[idx] = paged(q[idx], seq_index, kv_lens)
     return out

@@ -54,8 +54,8 @@ def test_forms(hd, hq, hkv, window, with_sinks, lens):
     assert prefill.usable(qkv, b, hd, window, sinks, qkv)
     want = _want(qkv, lens, hq, hkv, hd, window, sinks)
     _close(prefill.prefill_attention(qkv, b, hq, hkv, hd, window=window, sinks=sinks), want)
-    if hd == 128:
-        q = prefill.prefill_attention(qkv, b, hq, hkv, hd, window=window, sinks=sinks, quant_out=True)
+    if hd == 128 and not window and sinks is None:
+        q = prefill.prefill_attention(qkv, b, hq, hkv, hd, quant_out=True)
         got = q.data.view(torch.float8_e4m3fn).double() * q.scale.t().double().repeat_interleave(128, 1)
         assert (got - want).norm() / want.norm() < 2.0 ** -4
     assert ops.device_status(torch.device(DEV, 0)) == 0
