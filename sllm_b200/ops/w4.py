@@ -262,13 +262,21 @@ def _expandable(x, w: W4Weight, residual, tok_off, tok_scale, row_ptr) -> bool:
             and (residual is None or (residual.is_contiguous() and residual.dtype == torch.bfloat16 and residual.data_ptr() % 16 == 0)))
 
 
-def _linear_expanded(x: torch.Tensor, w: W4Weight, residual: Optional[torch.Tensor]) -> torch.Tensor:
-    """Rows of the weight are expanded to bf16 (exact) and multiplied on CTA pairs, EXPAND_ELEMENTS of them at a time."""
+def _expand_buffer(w: W4Weight, device) -> Optional[torch.Tensor]:
+    """Room for as many expanded rows as are multiplied at a time, held for the time of one product; None where the device has no such
+    memory left (an engine whose pages were sized to what was free)."""
+    try:
+        return torch.empty((min(w.n, max(256, EXPAND_ELEMENTS // w.k // 256 * 256)), w.k), dtype=torch.bfloat16, device=device)
+    except torch.OutOfMemoryError:
+        return None
+
+
+def _linear_expanded(x: torch.Tensor, w: W4Weight, residual: Optional[torch.Tensor], dense: torch.Tensor) -> torch.Tensor:
+    """Rows of the weight are expanded to bf16 (exact) and multiplied on CTA pairs, as many at a time as ``dense`` holds."""
     from .core import _p, _prompt_tile, _stream, workspace
     t, k = x.shape
     y = torch.empty((t, w.n), dtype=torch.bfloat16, device=x.device)
-    step = max(256, EXPAND_ELEMENTS // k // 256 * 256)
-    dense = torch.empty((min(step, w.n), k), dtype=torch.bfloat16, device=x.device)
+    step = dense.shape[0]
     lib, status = _lib.kernels(), _p(workspace(x.device).status)
     for r0 in range(0, w.n, step):
         rows = min(step, w.n - r0)
@@ -324,7 +332,10 @@ def linear_w4(x: torch.Tensor, w: W4Weight, residual: Optional[torch.Tensor] = N
     if w.groups > 1 and tok_off is None:
         raise ValueError("grouped weights need token offsets")
     if splits <= 0 and _expandable(x, w, residual, tok_off, tok_scale, row_ptr):
-        return _linear_expanded(x, w, residual)
+        dense = _expand_buffer(w, x.device)
+        if dense is not None:
+            return _linear_expanded(x, w, residual, dense)
+        # the packed kernel needs no room; without a K split its results have the same bits
     x = x.contiguous() if x.stride(1) != 1 or x.stride(0) % 8 else x
     y = torch.empty((t, w.n), dtype=torch.bfloat16, device=x.device)
     mgt = max_group_tokens or t

@@ -4,7 +4,7 @@ import pytest
 import torch
 
 from sllm_b200 import ops
-from sllm_b200.ops import w4
+from sllm_b200.ops import _lib, w4
 from sllm_b200.ops.w4 import W4Weight, linear_w4
 
 pytestmark = pytest.mark.gpu
@@ -38,6 +38,28 @@ def test_expanded_products_have_the_bits_of_packed_ones(fmt, t, n, k):
     r = torch.randn(t, n, generator=g, device=DEV).bfloat16()
     for res in (None, r):
         assert torch.equal(linear_w4(x, weight, residual=res), linear_w4(x, weight, residual=res, splits=1))
+
+
+def test_no_room_for_expanded_weights(monkeypatch):
+    """A product whose weight cannot be expanded for want of memory takes the packed kernel."""
+    g = torch.Generator(device=DEV).manual_seed(2)
+    weight = W4Weight.quantize_device("nvfp4", torch.randn(19200, 256, generator=g, device=DEV) * 0.05)
+    x = torch.randn(300, 256, generator=g, device=DEV).bfloat16()
+    want = linear_w4(x, weight)
+
+    def full(*a, **k):
+        raise torch.OutOfMemoryError("no room")
+
+    with monkeypatch.context() as m:
+        m.setattr(w4.torch, "empty", lambda *a, **k: full() if a[0] == (19200, 256) else torch.zeros(*a, **k))
+        _lib.dispatch_records(clear=True)
+        _lib.audit(True)
+        try:
+            got = linear_w4(x, weight)
+        finally:
+            _lib.audit(False)
+    assert [e["kernel"] for e in _lib.dispatch_records(clear=True)] == ["gemm_w4_kernel"]
+    assert torch.equal(got, want)
 
 
 @pytest.mark.parametrize("counts", [[0, 0, 300], [17, 0, 64, 65, 1, 128, 0, 129], [3] * 70, [0] * 40 + [200, 5]])
