@@ -558,11 +558,11 @@ SLLM_EXPORT int sllm_prefill_tile_rows(int hq, int hkv, int hd) {
 
 // tiles: device int32 [num_tiles][4] = {first token row of the sequence, sequence length, q0, 0}, q0 in steps of
 // sllm_prefill_tile_rows, ordered by the caller (most keys first).  qkv row stride is qkv_ld elements.  window: 0 or the number of
-// positions that a row sees; sinks: optional [hq].  E4M3 results (out_fp8, out_scale): heads of 128 without window and sinks.
+// positions that a row sees; sm_scale > 0; sinks: optional [hq].  E4M3 results (out_fp8, out_scale): heads of 128 without window and sinks.
 SLLM_EXPORT int sllm_prefill_attention(const void* qkv, int total_tokens, int qkv_ld, const int* tiles, int num_tiles,
                                        int hq, int hkv, int hd, int window, float sm_scale, const float* sinks, void* out_bf16,
                                        void* out_fp8, float* out_scale, int ld_scale, int* status, void* stream) {
-  if (!qkv || !tiles || num_tiles <= 0 || hq <= 0 || hkv <= 0 || hq % hkv || window < 0) return SLLM_ERR_INVALID_ARGUMENT;
+  if (!qkv || !tiles || num_tiles <= 0 || hq <= 0 || hkv <= 0 || hq % hkv || window < 0 || !(sm_scale > 0.f)) return SLLM_ERR_INVALID_ARGUMENT;
   if ((hd != 64 && hd != 128 && hd != 256) || (out_fp8 && (hd != 128 || window || sinks)))
     return SLLM_ERR_UNSUPPORTED_SHAPE;
   if (!out_bf16 && !(out_fp8 && out_scale)) return SLLM_ERR_INVALID_ARGUMENT;

@@ -18,20 +18,21 @@ MIN_TOKENS = 128
 TILE = 128
 
 
-def _heads_fit(q, hd, qkv) -> bool:
-    return (q.is_cuda and qkv is not None and qkv.dtype == torch.bfloat16 and hd in (64, 128, 256) and not _lib.fake_active()
+def _heads_fit(q, hd, qkv, sm_scale) -> bool:
+    # (the kernel masks scores ahead of their scale, which must not turn them round)
+    return ((sm_scale is None or sm_scale > 0) and q.is_cuda and qkv is not None and qkv.dtype == torch.bfloat16 and hd in (64, 128, 256) and not _lib.fake_active()
             and qkv.stride(1) == 1 and qkv.stride(0) == qkv.shape[1])
 
 
-def usable(q, batch, hd, window, sinks, qkv, quant_out: bool = False) -> bool:
+def usable(q, batch, hd, window, sinks, qkv, quant_out: bool = False, sm_scale: Optional[float] = None) -> bool:
     """Whether all rows of the batch take the kernel.  Results that are quantised to E4M3 are kept as they have been, since a last
     bit's difference moves them by a sixteenth: with a window or sinks they come from the pages."""
     if quant_out and (window or sinks is not None):
         return False
-    return batch.cu_seqlens_host is not None and batch.max_seqlen >= MIN_TOKENS and _heads_fit(q, hd, qkv)
+    return batch.cu_seqlens_host is not None and batch.max_seqlen >= MIN_TOKENS and _heads_fit(q, hd, qkv, sm_scale)
 
 
-def fresh_part(q, batch, hd, qkv) -> Optional[tuple]:
+def fresh_part(q, batch, hd, qkv, sm_scale: Optional[float] = None) -> Optional[tuple]:
     """(sequences that take the kernel, [lo, hi) runs of the other rows) of a batch that mixes prompts with running requests, or
     None where no prompt of MIN_TOKENS starts in it."""
     if batch.row_off_host is None or batch.starts_host is None:
@@ -49,7 +50,7 @@ def fresh_part(q, batch, hd, qkv) -> Optional[tuple]:
                 rest.append([off[i], off[i + 1]])
         batch.plans["fresh"] = (fresh, rest) if fresh else None
     part = batch.plans["fresh"]
-    return part if part is not None and batch.row_off_host[-1] == q.shape[0] and _heads_fit(q, hd, qkv) else None
+    return part if part is not None and batch.row_off_host[-1] == q.shape[0] and _heads_fit(q, hd, qkv, sm_scale) else None
 
 
 def build_tiles(cu_seqlens: list, device, rows: int = TILE, sequences: Optional[list] = None) -> torch.Tensor:

@@ -173,3 +173,19 @@ def test_rows_between_prompts_take_one_launch():
             _lib.audit(False)
         assert [e["kernel"] for e in _lib.dispatch_records(clear=True)] == ["prefill_attention_kernel", "paged_attention_kernel"]
         _close(got, want, 2)
+
+
+@pytest.mark.parametrize("scale", [0.0, -0.2, 0.2])
+@pytest.mark.parametrize("hd,window", [(64, 0), (128, 0), (128, 50), (256, 0)])
+def test_any_scale(scale, hd, window):
+    """Scores may be turned round or levelled by their scale."""
+    hq, hkv, page, lens = 4, 2, 16, [200, 33]
+    g = torch.Generator(device=DEV).manual_seed(hd)
+    kv = KVLayer(*(torch.zeros(26, hkv, page, hd, device=DEV).bfloat16() for _ in range(2)), None, None, False, page)
+    b = make_prefill_batch([[0] * n for n in lens], torch.arange(26, dtype=torch.int32, device=DEV).view(2, 13), DEV)
+    qkv = torch.randn(sum(lens), (hq + 2 * hkv) * hd, generator=g, device=DEV).bfloat16()
+    q = ops.rope_kv_append(qkv, b.positions, b.seq_index, b.block_table, kv, hq, hkv, hd, 1e4)
+    got = ops.attention(q, kv, b, hq, hkv, hd, qkv=qkv, window=window, sm_scale=scale)
+    turned = qkv.double()
+    turned[:, :hq * hd] *= scale * math.sqrt(hd)
+    _close(got, _want(turned, lens, hq, hkv, hd, window, None))
