@@ -27,7 +27,7 @@ def _heads_fit(q, hd, qkv, sm_scale) -> bool:
 def usable(q, batch, hd, window, sinks, qkv, quant_out: bool = False, sm_scale: Optional[float] = None) -> bool:
     """Whether all rows of the batch take the kernel.  Results that are quantised to E4M3 are kept as they have been, since a last
     bit's difference moves them by a sixteenth: with a window or sinks they come from the pages."""
-    if quant_out and (window or sinks is not None):
+    if quant_out and (window or sinks is not None or hd != 128):
         return False
     return batch.cu_seqlens_host is not None and batch.max_seqlen >= MIN_TOKENS and _heads_fit(q, hd, qkv, sm_scale)
 

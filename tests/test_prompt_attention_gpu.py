@@ -189,3 +189,14 @@ def test_any_scale(scale, hd, window):
     turned = qkv.double()
     turned[:, :hq * hd] *= scale * math.sqrt(hd)
     _close(got, _want(turned, lens, hq, hkv, hd, window, None))
+
+
+@pytest.mark.parametrize("hd", [64, 256])
+def test_quantised_results_of_other_heads_are_refused(hd):
+    """As by the pages, which need heads of 128 for them."""
+    hq, hkv, n = 4, 2, 200
+    kv = KVLayer(*(torch.zeros(13, hkv, 16, hd, device=DEV).bfloat16() for _ in range(2)), None, None, False, 16)
+    b = make_prefill_batch([[0] * n], torch.arange(13, dtype=torch.int32, device=DEV).view(1, 13), DEV)
+    qkv = torch.zeros(n, (hq + 2 * hkv) * hd, dtype=torch.bfloat16, device=DEV)
+    with pytest.raises(ValueError):
+        ops.attention(qkv[:, :hq * hd], kv, b, hq, hkv, hd, qkv=qkv, quant_out=True)
