@@ -163,12 +163,13 @@ def _linear_prompt(x: torch.Tensor, w: LinearWeight, y: torch.Tensor, scale_x: O
     scaled = scale_x is not None
     epilogue = 1 if residual is not None else {None: 0, "relu_sq": 2, "softcap": 3}[act]
     bn = _prompt_tile(m, n, scaled)
+    # (a scale matrix of one K block may have any leading stride)
     if _lib.audit_enabled():
         _lib.record_dispatch("linear", "gemm_prompt_kernel", m=m, n=n, k=k, kind=w.kind, bn=bn,
                              grid=[min(148, 2 * ((m + 255) // 256) * ((n + bn - 1) // bn))])
     rc = _lib.kernels().sllm_gemm_prompt(_p(x), _p(w.w), _p(y), _p(scale_x), _p(w.scale_t) if scaled else None, _p(residual), m, n, k,
-                                         x.stride(0), y.stride(0), scale_x.stride(0) if scaled else 0,
-                                         w.scale_t.stride(0) if scaled else 0, epilogue, act_arg, None, 1 if scaled else _GEMM_PARTS, 1, bn,
+                                         x.stride(0), y.stride(0), *(max(s.stride(0), s.shape[1]) if scaled else 0 for s in (scale_x, w.scale_t)),
+                                         epilogue, act_arg, None, 1 if scaled else _GEMM_PARTS, 1, bn,
                                          _p(workspace(x.device).status), _stream())
     _lib.check(rc, "gemm_prompt")
 

@@ -77,3 +77,14 @@ def test_a_soft_cap_that_is_not_positive_is_refused(m, cap):
     x, w, _, _, _ = _operands(m, 64, 64, False, 1)
     with pytest.raises(ops.KernelError):
         ops.linear(x, w, act="softcap", act_arg=cap)
+
+
+@pytest.mark.parametrize("m", [128, 129, 300])
+@pytest.mark.parametrize("k", [64, 128])
+def test_scales_of_one_block_with_any_leading_stride(m, k):
+    """One K block: the transposed scales of a file are [1, n] with a leading stride of 1."""
+    x, w, xf, wf, _ = _operands(m, 72, k, True, k)
+    turned = lambda s: torch.empty(s.shape[1], 1, device=DEV).copy_(s.t()).t().contiguous()
+    xt, wt = ops.QTensor(x.data, turned(x.scale)), LinearWeight("fp8", w.w, turned(w.scale_t))
+    assert xt.scale.stride(0) == 1 and wt.scale_t.stride(0) == 1
+    _close(ops.linear(xt, wt), xf @ wf.t(), xf, wf)
