@@ -4,6 +4,7 @@
     python -m sllm_b200.utils.kernel_bench --op attention --batch 32 --ctx 2048
     python -m sllm_b200.utils.kernel_bench --op prefill --seqs 4 --len 2048
     python -m sllm_b200.utils.kernel_bench --op decode-gemms --m 32 --graph
+    python -m sllm_b200.utils.kernel_bench --op prompt-kernels            # the ops that prompts consist of, one line each
 
 Timing follows the usual hygiene: warm-up, an L2 flush (a 256 MB write) before each timed launch, CUDA
 events on the launching stream, median of the repetitions.  Fractions are reported against the
@@ -213,9 +214,60 @@ def bench_prefill(seqs, length, hq, hkv, reps):
             "TFLOPs": flops / t / 1e12, "fraction": flops / fl / t, "fraction_basis": tag}
 
 
+def bench_prompt_kernels(reps):
+    """(op, size, seconds, operations) of the ops that prompts consist of, each through its public call."""
+    from ..engine.batch import make_prefill_batch
+    from ..ops import delta, gdn
+    dev = "cuda"
+    rnd = lambda *shape: torch.randn(*shape, device=dev).bfloat16()
+
+    for m, n, k in ((130, 4096, 4096), (527, 6144, 4096), (1500, 2048, 9216), (5400, 4096, 14336), (8192, 28672, 4096)):
+        x, w = rnd(m, k), rnd(n, k) * 0.02
+        xq, wq = ops.quant_fp8(x), ops.quant_fp8(w)
+        dense, fp8 = LinearWeight("dense", w), LinearWeight("fp8", wq.data, wq.scale)
+        yield "linear bf16", f"{m} x {n} x {k}", timed(lambda: ops.linear(x, dense), reps), 2.0 * m * n * k
+        yield "linear E4M3", f"{m} x {n} x {k}", timed(lambda: ops.linear(xq, fp8), reps), 2.0 * m * n * k
+
+    def batch(lens):
+        blocks = (max(lens) + 15) // 16
+        table = torch.arange(len(lens) * blocks, dtype=torch.int32, device=dev).view(len(lens), blocks)
+        return make_prefill_batch([[0] * n for n in lens], table, dev), len(lens) * blocks
+
+    for lens, hq, hkv, hd, window, quant in (([8192], 32, 8, 128, 0, False), ([8192], 32, 8, 128, 0, True), ([2048, 782], 16, 4, 256, 0, False),
+                                             ([1000, 536, 823], 64, 8, 64, 0, False), ([1000, 536, 823], 64, 8, 64, 128, False)):
+        b, pages = batch(lens)
+        kv = KVLayer(rnd(pages, hkv, 16, hd), rnd(pages, hkv, 16, hd), None, None, False, 16)
+        qkv = rnd(sum(lens), (hq + 2 * hkv) * hd)
+        size = f"{'+'.join(map(str, lens))} tokens, {hq} + 2 x {hkv} heads x {hd}" + (f", window {window}" if window else "") + (", E4M3" if quant else "")
+        seen = sum(n * (n + 1) // 2 if not window else sum(min(i + 1, window) for i in range(n)) for n in lens)
+        if hd == 128 and not quant:
+            yield "rotation and pages", size, timed(lambda: ops.rope_kv_append(qkv, b.positions, b.seq_index, b.block_table, kv, hq, hkv, hd, 1e4), reps), 0
+        yield "attention", size, timed(lambda: ops.attention(qkv[:, :hq * hd], kv, b, hq, hkv, hd, qkv=qkv, window=window, quant_out=quant),
+                                       reps), 4.0 * hq * hd * seen
+
+    lens, qk, vh = [2048, 782], 16, 32
+    t, b = sum(lens), batch(lens)[0]
+    slots = torch.tensor([1, 0], dtype=torch.int32, device=dev)
+    width = (2 * qk + vh) * 128
+    x, taps, hist = rnd(t, width), rnd(width, 4), rnd(2, 3, width)
+    yield "convolution (gated delta net)", f"2048+782 rows x {width}", timed(lambda: gdn.conv_silu(x, taps, hist, b.row_off, slots), reps), 0
+    z, gates, state = rnd(t, vh * 128), rnd(t, 2 * vh), torch.zeros(2, vh, 128, 128, device=dev)
+    vec = [rnd(vh).float(), rnd(vh), rnd(128).float()]
+    yield "gated delta rule", f"2048+782 tokens, {vh} heads", timed(
+        lambda: gdn.recurrent(x, z, gates[:, :vh], gates[:, vh:], *vec, state, b.row_off, slots, qk, vh), reps), 0
+
+    t, heads, dim, rank = 1500, 16, 128, 64
+    spec, n = delta.DeltaSpec(heads, dim, rank), heads * dim
+    proj, w2 = rnd(t, 5 * n + rank), LinearWeight("dense", rnd(n, rank) * 0.1)
+    vecs, state = [rnd(n).float() for _ in range(3)], torch.zeros(1, heads, dim, dim, device=dev)
+    off, slot = torch.tensor([0, t], dtype=torch.int32, device=dev), torch.zeros(1, dtype=torch.int32, device=dev)
+    yield "generalised delta rule", f"{t} tokens, {heads} heads x {dim}", timed(
+        lambda: delta.general_delta(proj, spec, w2, *vecs, 1e-5, state, off, slot, False), reps), 0
+
+
 def main():
     ap = argparse.ArgumentParser()
-    ap.add_argument("--op", required=True, choices=["gemm", "gemm-w4", "attention", "prefill", "decode-gemms"])
+    ap.add_argument("--op", required=True, choices=["gemm", "gemm-w4", "attention", "prefill", "decode-gemms", "prompt-kernels"])
     ap.add_argument("--fmt", default="nvfp4", choices=["nvfp4", "mxfp4"])
     ap.add_argument("--groups", type=int, default=1)
     ap.add_argument("--active", type=int, default=0, help="gemm-w4, grouped: groups that receive tokens (0 = all)")
@@ -244,6 +296,9 @@ def main():
         print(json.dumps(bench_attention(a.batch, a.ctx, a.hq, a.hkv, a.hd, a.fp8, a.reps, a.graph)))
     elif a.op == "prefill":
         print(json.dumps(bench_prefill(a.seqs, a.len, a.hq, a.hkv, a.reps)))
+    elif a.op == "prompt-kernels":
+        for op, size, t, flops in bench_prompt_kernels(a.reps):
+            print(json.dumps({"op": op, "size": size, "us": round(t * 1e6, 1), **({"TFLOPs": round(flops / t / 1e12, 1)} if flops else {})}))
     else:
         for (n, k) in ((6144, 4096), (4096, 4096), (28672, 4096), (4096, 14336), (128256, 4096)):
             print(json.dumps(bench_gemm(a.m, n, k, True, a.reps, a.graph)))
