@@ -22,12 +22,13 @@
 //
 // Measured (B200, one launch, m x n x k, us; before: the 128 x 128 tiles of gemm_tcgen05.cu):
 //                          bf16 before -> now             E4M3 before -> now
-//   130 x 4096 x 4096          38 ->   31                     38 ->   25
-//   527 x 6144 x 4096          70 ->   38                     58 ->   46
-//   1500 x 2048 x 9216        129 ->   61                    106 ->   83
-//   5400 x 4096 x 14336       910 ->  418                    732 ->  564
-//   8192 x 28672 x 4096      3060 -> 1197 (1.61 PFLOP/s)    2497 -> 1620 (1.19 PFLOP/s)
-// (bf16 in one chain per tile, which is less exact: 29, 36, 59, 408, 1195 us in the same run)
+//   130 x 4096 x 4096          38 ->   31                     32 ->   25
+//   527 x 6144 x 4096          71 ->   39                     58 ->   47
+//   1500 x 2048 x 9216        129 ->   61                    106 ->   84
+//   5400 x 4096 x 14336       909 ->  426                    736 ->  565
+//   8192 x 28672 x 4096      3060 -> 1227 (1.57 PFLOP/s)    2500 -> 1634 (1.18 PFLOP/s)
+// (bf16 in one chain per tile, which is less exact: 30, 35, 57, 414, 1220 us; with L2 warm the second takes 29.4 and 30.7.  The largest
+// E4M3 product takes up to 2250 us right behind others of its size, when the power limit holds the clock.)
 // bf16 with 256 columns keeps the tensor pipe 96 % active (4096 x 14336 x 4096); narrower tiles are held by operands out of L2.  E4M3
 // spends about 2000 cycles a K block in the promotion (pipe 26 % active); reading 128 x 256 sums out of tensor memory alone takes 560.
 #include "pair_mma.cuh"
@@ -55,17 +56,15 @@ struct GpShape {
   static constexpr bool kMoveRegs = kThreads == 384;
   static constexpr int kOutBytes = 4 * kGroups * 4096;     // 32 rows x 64 columns per epilogue warp
   static constexpr int kScaleBytes = kScaled ? kGpScaleRing * kGpScaleChunk * (kGpRows + BN) * 4 : 0;
-  // accumulators: two of every partial sum that is under way; scaled: of K blocks in turn
-  static constexpr int kLive = kScaled || BN == 256 ? 1 : BN == 128 ? 2 : 4;
-  static constexpr int kAcc = kScaled && BN < 256 ? 4 : 2 * kLive;
+  static constexpr int kAcc = BN < 256 ? 4 : 2;            // accumulators: of partial sums in turn; scaled: of K blocks
   static constexpr uint32_t kTmem = kAcc * BN;
 };
 
 struct __align__(16) GpShared {
   uint64_t full[kGpMaxStages];              // first CTA's: the bytes of both
   uint64_t empty[kGpMaxStages];
-  uint64_t acc_full[8];
-  uint64_t acc_empty[8];                    // first CTA's: the epilogue warps of both
+  uint64_t acc_full[4];
+  uint64_t acc_empty[4];                    // first CTA's: the epilogue warps of both
   uint64_t scale_full[kGpScaleRing];
   uint64_t scale_empty[kGpScaleRing];
   uint32_t tmem_base;
@@ -96,29 +95,15 @@ __device__ __forceinline__ void gp_tile(const GpParams& p, int t, int& tm, int& 
   tn = g * kGpGroupN + r - tm * wide;
 }
 
-// The K blocks of a tile in the order that they are multiplied: kLive partial sums at a time, whose blocks come in turn (neighbours
-// along K share DRAM and L2 lines; 130 x 4096 x 4096 takes 32.8 us with one partial sum after the other, 30.7 with both at a time).
-template <int kLive>
+// The K blocks of a tile in the order that they are multiplied: those of partial sum 0, of partial sum 1, ..  (Two at a time, so that
+// neighbours along K follow one another, took as long.)
 struct GpBlocks {
-  int kb = 0, part = 0, lo = 0, hi;                        // partial sums [lo, hi) are under way
-  __device__ __forceinline__ explicit GpBlocks(const GpParams& p) : hi(min(kLive, p.parts)) {}
+  int kb = 0, part = 0;
   __device__ __forceinline__ bool first() const { return kb == part; }
   __device__ __forceinline__ bool last(const GpParams& p) const { return kb + p.parts >= p.num_kb; }
   __device__ __forceinline__ void next(const GpParams& p) {
-    if constexpr (kLive == 1) {
-      kb += p.parts;
-      if (kb >= p.num_kb) kb = ++part;
-      return;
-    }
-    ++kb;
-    if (++part == hi) {
-      kb += p.parts - (hi - lo);
-      part = lo;
-    }
-    if (kb >= p.num_kb) {
-      kb = part = lo = hi;
-      hi = min(lo + kLive, p.parts);
-    }
+    kb += p.parts;
+    if (kb >= p.num_kb) kb = ++part;
   }
 };
 
@@ -180,7 +165,7 @@ gemm_prompt_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
         gp_tile(p, pair, tm, tn);
         const int pre = min(p.num_kb, S::kStages);
         if (!p.w_const) pdl_wait();
-        GpBlocks<S::kLive> first(p);
+        GpBlocks first;
         for (int i = 0; i < pre; ++i, first.next(p)) {
           if (rank == 0) mbar_expect_tx(&sh->full[i], 2 * S::kStage);
           load_w(i, first.kb, tn);
@@ -190,7 +175,7 @@ gemm_prompt_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
         bool ok = true;
         for (int t = pair; ok && t < tiles; t += pairs) {
           gp_tile(p, t, tm, tn);
-          GpBlocks<S::kLive> b(p);
+          GpBlocks b;
           for (int i = 0; i < p.num_kb; ++i, ++it, b.next(p)) {
             const int s = it % S::kStages;
             if (it >= pre) {
@@ -216,15 +201,15 @@ gemm_prompt_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
     } else if (warp == 1) {
       if (rank == 0) {
         constexpr uint32_t idesc = make_idesc(kScaled ? kFmtE4M3 : kFmtBf16, 256, BN);
-        int it = 0, acc = 0;                               // acc: accumulators handed over by earlier tiles (scaled: blocks)
+        int it = 0, acc = 0;                               // acc: accumulators handed over so far
         bool ok = true;
         for (int t = pair; ok && t < tiles; t += pairs) {
-          GpBlocks<S::kLive> b(p);
+          GpBlocks b;
           for (int i = 0; i < p.num_kb; ++i, ++it, b.next(p)) {
-            const int s = it % S::kStages, use = kScaled ? acc : acc + b.part, buf = use % S::kAcc;
+            const int s = it % S::kStages, buf = acc % S::kAcc;
             ok = mbar_wait(&sh->full[s], (it / S::kStages) & 1, abort_flag, p.status, SLLM_DEV_TIMEOUT_TMA_FULL);
             if (ok && (kScaled || b.first()))
-              ok = mbar_wait(&sh->acc_empty[buf], ((use / S::kAcc) & 1) ^ 1, abort_flag, p.status, SLLM_DEV_TIMEOUT_TMEM_EMPTY);
+              ok = mbar_wait(&sh->acc_empty[buf], ((acc / S::kAcc) & 1) ^ 1, abort_flag, p.status, SLLM_DEV_TIMEOUT_TMEM_EMPTY);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             tc_fence_after();
@@ -239,9 +224,8 @@ gemm_prompt_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_consta
               if (last) pair_commit(&sh->acc_full[buf]);
             }
             __syncwarp();
-            if (kScaled) ++acc;
+            acc += last;
           }
-          if (!kScaled) acc += p.parts;
         }
       }
     } else if (kScaled) {
@@ -460,8 +444,8 @@ using namespace sllm;
 // x [m, k] (row stride ldx elements), w [n, k] contiguous, y [m, n] bf16 (row stride ldy): bf16 operands, or with scale_x / scale_w
 // E4M3 and scales [ceil(k / 128), ld].  epilogue: 0 store, 1 add residual [m, ldy], 2 square of relu, 3 act_arg tanh(. / act_arg).
 // alpha: optional device scalar that multiplies the sums of bf16 operands.  parts: partial sums of bf16 operands, 1 to 4 (K blocks of 64
-// taken in turn).  w_const: no kernel of the stream writes w.  bn: columns of a pair's tile, 64, 128 or 256.  n and ldy are multiples
-// of 8, rows of x and w of 16 bytes.
+// taken in turn).  w_const: no kernel of the stream writes w.  bn: columns of a pair's tile, 128, 256 or (scaled) 64.  n and ldy
+// are multiples of 8, rows of x and w of 16 bytes.
 SLLM_EXPORT int sllm_gemm_prompt(const void* x, const void* w, void* y, const float* scale_x, const float* scale_w, const void* residual,
                                  int m, int n, int k, long long ldx, int ldy, int ld_sx, int ld_sw, int epilogue, float act_arg,
                                  const float* alpha, int parts, int w_const, int bn, int* status, void* stream) {
@@ -480,7 +464,7 @@ SLLM_EXPORT int sllm_gemm_prompt(const void* x, const void* w, void* y, const fl
   p.scale_x = scale_x; p.scale_w = scale_w; p.residual = static_cast<const __nv_bfloat16*>(residual); p.status = status;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   switch (bn) {
-    case 64: return scaled ? gemm_prompt_go<64, true>(x, w, y, ldx, k, p, st) : gemm_prompt_go<64, false>(x, w, y, ldx, k, p, st);
+    case 64: return scaled ? gemm_prompt_go<64, true>(x, w, y, ldx, k, p, st) : SLLM_ERR_UNSUPPORTED_SHAPE;
     case 128: return scaled ? gemm_prompt_go<128, true>(x, w, y, ldx, k, p, st) : gemm_prompt_go<128, false>(x, w, y, ldx, k, p, st);
     case 256: return scaled ? gemm_prompt_go<256, true>(x, w, y, ldx, k, p, st) : gemm_prompt_go<256, false>(x, w, y, ldx, k, p, st);
     default: return SLLM_ERR_INVALID_ARGUMENT;

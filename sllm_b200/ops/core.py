@@ -140,19 +140,17 @@ def _gemm_plan(m: int, n: int, k_blocks: int):
 
 
 # Cycles of one 128-byte K block of a pair's tile by its columns (csrc/gemm_prompt.cu), measured with the machine full: bf16 is held
-# by L2 below 256 columns and by the tensor cores there, E4M3 by the promotion of every block's sums
-_PROMPT_BLOCK = {False: {64: 520, 128: 540, 256: 700}, True: {64: 830, 128: 1060, 256: 2050}}
-
-
+# by L2 below 256 columns and by the tensor cores there, E4M3 by the promotion of every block's sums.  (bf16 in 64 columns took 550.)
+_PROMPT_BLOCK = {False: {128: 540, 256: 700}, True: {64: 830, 128: 1060, 256: 2050}}
 _GEMM_PARTS = 2            # partial sums of a bf16 product (two issuers of the 128-column tiles in csrc/gemm_tcgen05.cu)
 
 
 def _prompt_tile(m: int, n: int, scaled: bool) -> int:
     """Columns of a tile of the prompt product: the fewest cycles over the waves of 74 CTA pairs, 256 rows a pair.  Narrow tiles
-    spread few rows over more pairs (130 x 4096 x 4096: 25 us with 64 columns, 31 with 256), wide ones reuse their operands
-    (8192 x 28672 x 4096: 2310 us with 64, 1190 with 256)."""
+    spread few rows over more pairs (bf16, 130 x 4096 x 4096: 29.7 us with 128 columns, 33.8 with 256), wide ones reuse their operands
+    (8192 x 28672 x 4096: 1830 us with 128, 1200 with 256)."""
     cost = _PROMPT_BLOCK[scaled]
-    return min((256, 128, 64), key=lambda bn: (((m + 255) // 256 * ((n + bn - 1) // bn) + 73) // 74) * cost[bn])
+    return min(sorted(cost, reverse=True), key=lambda bn: (((m + 255) // 256 * ((n + bn - 1) // bn) + 73) // 74) * cost[bn])
 
 
 def _linear_prompt(x: torch.Tensor, w: LinearWeight, y: torch.Tensor, scale_x: Optional[torch.Tensor], residual: Optional[torch.Tensor],

